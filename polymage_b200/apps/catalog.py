@@ -93,8 +93,8 @@ LAPLACIAN = dict(tile_sizes=(32, 64), group_size=10,
 # grid, 10 pre-smoothings and none after or on the coarsest level
 # (multigrid/jacobi{2D,3D}/Makefile:10-16), NAS MG class W (NAS-PB-MG-3.2/
 # Makefile:9), interpolation of a 2048x2048 RGBA image.
-INTERPOLATE = dict(rows=2048, cols=2048, tile_sizes=(32, 64), group_size=11,
-                   options=('min_blocks=3',))
+INTERPOLATE = dict(rows=2048, cols=2048, tile_sizes=(16, 64), group_size=11,
+                   options=('channel_tile_all',))
 JACOBI2D = dict(N=2048, T=10, tile_sizes=(32, 64), group_size=5,
                 options=('stage_pointwise',))
 JACOBI3D = dict(N=128, T=10, tile_sizes=(8, 16, 32), group_size=1,

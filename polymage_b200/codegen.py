@@ -65,7 +65,7 @@ from .expression import substitute_vars, getType, affine_form
 from .bounds import part_boxes
 from .pipe import body_parts
 from .tiling import is_data_dependent
-from .evaluate import monotone_dir, is_min_max
+from .evaluate import EvalError, eval_int, monotone_dir, is_min_max
 
 _INT_T = (C.Int, C.UInt, C.Short, C.UShort, C.Char, C.UChar, C.Long,
           C.ULong)
@@ -180,6 +180,13 @@ class ExprCtx(object):
         # as its unclamped arm (only inside index expressions)
         self.fold_clamps = False
         self._in_index = 0
+        # region inference of border tiles: integer division rounds down
+        # (a region may start left of its domain, where C's truncation
+        # would move its origin)
+        self.floor_div = False
+        # name of a subexpression of parameters only that the launch
+        # carries precomputed (set by the group generators)
+        self.hoist = None
 
     def temp(self):
         self.ntemp += 1
@@ -242,6 +249,8 @@ class ExprCtx(object):
             args = [_subst(a, bind) for a in e.arguments]
             return self.reader(e.objectRef, args, self)
         if isinstance(e, AbstractBinaryOpNode):
+            if self.hoist is not None and _uniform_quotient(e):
+                return self.hoist(e)
             if e.op == '%':
                 sm = self._static_mod(e, bind)
                 if sm is not None:
@@ -250,6 +259,8 @@ class ExprCtx(object):
                 sd = self._static_div(e, bind)
                 if sd is not None:
                     return sd
+                if self.floor_div:
+                    return self._floor_div(e, bind)
             if e.op in ('/', '%') and self._unsigned_ok(e, bind):
                 # truncating division of a non-negative int by a positive
                 # constant equals unsigned division (a shift or mask for
@@ -330,6 +341,13 @@ class ExprCtx(object):
         return {C.Pow: 'pow', C.Powf: 'powf', C.Log: 'log', C.Exp: 'exp',
                 C.Sin: 'sin', C.Cos: 'cos', C.Sqrt: 'sqrt', C.Sqrtf: 'sqrtf',
                 C.Abs: 'pm_abs'}[type(e)]
+
+    def _floor_div(self, e, bind):
+        k = _const_int(e.right)
+        a = self.expr(e.left, bind)
+        if k is not None and k > 0 and k & (k - 1) == 0:
+            return "((%s) >> %d)" % (a, k.bit_length() - 1)
+        return "pm_floordiv(%s, %s)" % (a, self.expr(e.right, bind))
 
     def _unsigned_ok(self, e, bind):
         if not self.var_lo:
@@ -579,6 +597,107 @@ def _has_clamp(e):
             return True
         if hasattr(n, 'children'):
             stack.extend(n.children())
+    return False
+
+
+def _uniform_quotient(e):
+    """Whether ``e`` is floating-point arithmetic on parameters and
+    literals with a division in it."""
+    def ok(x):
+        """(arithmetic on parameters and literals, divides floats)"""
+        x = Value.numericToValue(x)
+        if isinstance(x, (Value, C.Parameter)):
+            return True, False
+        if isinstance(x, AbstractUnaryOpNode):
+            return ok(x.child)
+        if isinstance(x, AbstractBinaryOpNode) and x.op in '+-*/':
+            a, b = ok(x.left), ok(x.right)
+            return a[0] and b[0], a[1] or b[1] or (
+                x.op == '/' and a[0] and b[0] and
+                getType(x) in (C.Float, C.Double))
+        return False, False
+    return ok(e) == (True, True)
+
+
+def _clamps(e):
+    """(arm, bound, is_min) of every clamp ``min/max(arm, bound)`` in an
+    index."""
+    out = []
+    stack = [e]
+    while stack:
+        n = stack.pop()
+        arm = _clamp_arm(n)
+        if arm is not None:
+            t, f, c = n.true_expression, n.false_expression, n.condition
+            less = c.conditional in ('<', '<=')
+            straight = (str(c.lhs), str(c.rhs)) == (str(t), str(f))
+            out.append((arm, f if arm is t else t, less == straight))
+        if hasattr(n, 'children'):
+            stack.extend(n.children())
+    return out
+
+
+def _strip_clamps(e):
+    """Index ``e`` with its clamps replaced by their arms."""
+    arm = _clamp_arm(e)
+    if arm is not None:
+        return _strip_clamps(arm)
+    if isinstance(e, AbstractBinaryOpNode):
+        a, b = _strip_clamps(e.left), _strip_clamps(e.right)
+        return {'+': lambda: a + b, '-': lambda: a - b,
+                '*': lambda: a * b, '/': lambda: a / b}[e.op]()
+    return e
+
+
+class _ArmFn(object):
+    """The arm of a clamp inside index function ``fn``."""
+
+    def __init__(self, fn, arm):
+        self.kind = 'mono'
+        self.expr, self.var, self.cdim = arm, fn.var, fn.cdim
+
+
+def _fold(op, terms, empty):
+    """``op(t0, op(t1, ...))`` in C text."""
+    if not terms:
+        return empty
+    out = terms[-1]
+    for t in reversed(terms[:-1]):
+        out = "%s(%s, %s)" % (op, t, out)
+    return out
+
+
+def _linear(e):
+    """({term text: coefficient}, constant) of an integer bound, with
+    what is not affine (``C / 2``) as a term of its own."""
+    e = Value.numericToValue(e)
+    f = affine_form(e)
+    if f is not None:
+        return dict((str(k), c) for k, c in f[0].items()), f[1]
+    if isinstance(e, AbstractBinaryOpNode) and e.op in '+-':
+        p, q = _linear(e.left), _linear(e.right)
+        s = 1 if e.op == '+' else -1
+        co = dict(p[0])
+        for k, c in q[0].items():
+            co[k] = co.get(k, 0) + s * c
+        return dict((k, c) for k, c in co.items() if c), p[1] + s * q[1]
+    if isinstance(e, AbstractUnaryOpNode) and e.op == '-':
+        p = _linear(e.child)
+        return dict((k, -c) for k, c in p[0].items()), -p[1]
+    return {str(e): 1}, 0
+
+
+def _boxes_disjoint(a, b, variables):
+    """Whether two boxes provably have no common point: along some
+    variable a lower bound of one exceeds an upper bound of the other by a
+    constant."""
+    def above(l, h):
+        p, q = _linear(l), _linear(h)
+        return p[0] == q[0] and p[1] > q[1]
+    for v in variables:
+        for p, q in ((a, b), (b, a)):
+            if any(above(l, h) for l in p.lo[v] for h in q.hi[v]):
+                return True
     return False
 
 
@@ -1737,7 +1856,6 @@ class StencilGen(object):
 
     def __init__(self, pg, group):
         self.pg = pg
-        self.fast = False
         self.clamp = False
         self.inside = False
         self.has_inside = False
@@ -1787,6 +1905,8 @@ class StencilGen(object):
         w.open("struct __align__(64) %s_desc" % k)
         for n in stage_nodes:
             w("CUtensorMap tm_%s;" % self.node_name(n))
+        hoist_decl = len(w.lines)
+        self.hoisted = {}
         for prm in pg.params:
             w("%s %s;" % (pg.ptype(prm), pg.pmap[prm]))
         for f in bufs:
@@ -1807,9 +1927,25 @@ class StencilGen(object):
         w("int stride;          // no queue: a CTA's tiles are gridDim.x apart")
         w.close("};")
         w("")
+        self.hoist_uses = []
         self.gen_kernel()
+        # scalars of parameters that the kernel divides with: computed once
+        # per call on the host instead of once per thread and tile (a
+        # double division is some 40 dependent instructions)
+        for i in sorted(self.hoist_uses, reverse=True):
+            w.lines[i:i] = ["    const %s %s = D.%s;" % (t, h, h)
+                            for t, h, _ in self.hoisted.values()]
+        w.lines[hoist_decl:hoist_decl] = [
+            "  %s %s;" % (t, h) for t, h, _ in self.hoisted.values()]
         self.gen_launcher()
         self.gen_footprint()
+
+    def hoist(self, e):
+        key = str(e)
+        if key not in self.hoisted:
+            t = "double" if getType(e) is C.Double else "float"
+            self.hoisted[key] = (t, "h_%d" % len(self.hoisted), e)
+        return self.hoisted[key][1]
 
     def gen_footprint(self):
         """Host function ``<k>_footprint(D, tile, in_end, a_lo, a_hi)``: the
@@ -1868,8 +2004,8 @@ class StencilGen(object):
             w.close()
         an = self.node_name(plan.node_of[plan.anchor])
         for d in range(na):
-            w("a_lo[%d] = r_%s_lo%d; a_hi[%d] = r_%s_hi%d;" % (d, an, d, d, an,
-                                                              d))
+            w("a_lo[%d] = pm_imax(a_lo%d, d_%s_lo%d); a_hi[%d] = pm_imin("
+              "a_hi%d, d_%s_hi%d);" % (d, d, an, d, d, d, an, d))
         w.close()
         w("")
         pg.w = saved_w
@@ -2040,7 +2176,9 @@ class StencilGen(object):
           "%s);" % tile)
         w("const %s_desc& D = *Dp;" % k)
         pg.declare_params(w, "D")
+        self.hoist_uses.append(len(w.lines))
         ctx = ExprCtx(w, 'device', pg.pmap, self.reader)
+        ctx.hoist = self.hoist
         self.ctx = ctx
         # tile coordinates
         w("int rem = %s - D.tile_base;" % tile)
@@ -2120,95 +2258,188 @@ class StencilGen(object):
               % (t, nm, t, n.smem_off, buf, self.plan.stage_delta))
             self.decl_smem_origin(n)
 
-    def empty_expr(self, n, kind="r"):
+    def empty_expr(self, n):
         nm = self.node_name(n)
-        return " || ".join("%s_%s_lo%d > %s_%s_hi%d" % (kind, nm, d, kind,
-                                                        nm, d)
+        return " || ".join("r_%s_lo%d > r_%s_hi%d" % (nm, d, nm, d)
                            for d in range(n.ndims))
 
+    def const_dim(self, f, d):
+        """Whether dimension ``d`` of ``f`` has an extent free of
+        parameters (channels, a grid's intensity bins)."""
+        from .tiling import _const_extent
+        key = (id(f), d)
+        memo = self.pg.__dict__.setdefault('_const_dims', {})
+        if key not in memo:
+            memo[key] = _const_extent(f.domain[d],
+                                      self.pg.p.int_env()) is not None
+        return memo[key]
+
+    def use_bounds(self, m, d):
+        """Bounds (C text) of the points of consumer ``m`` along its
+        dimension ``d`` that its producers' regions are inferred from: its
+        region, in a dimension of constant extent also inside its Case
+        box's constant bounds."""
+        nm = self.node_name(m)
+        lo, hi = "r_%s_lo%d" % (nm, d), "r_%s_hi%d" % (nm, d)
+        cb = getattr(m, 'case_box', None)
+        if cb and self.const_dim(m.func, d):
+            for e in cb[d][0]:
+                if _const_int(e) is not None:
+                    lo = "pm_imax(%s, %d)" % (lo, _const_int(e))
+            for e in cb[d][1]:
+                if _const_int(e) is not None:
+                    hi = "pm_imin(%s, %d)" % (hi, _const_int(e))
+        return lo, hi
+
     def gen_regions(self):
+        """The region of every node for the tile: ``r_<node>_lo/hi``.
+
+        Regions are not clamped to the image: along a parametric dimension
+        a region keeps its interior extent on every tile and may reach
+        past its domain, so each buffer has the same layout and the same
+        origin residues on border tiles as on interior ones (TMA and the
+        cooperative loads fill what lies outside with zeros, and no point
+        whose Case holds reads it).  Clamped taps count with their
+        unclamped index: a clamp moves an index towards the domain, which
+        the region intersects, so never out of the region.  Along a
+        dimension of constant extent regions stay inside the domain."""
         pg = self.pg
         plan = self.plan
         w = pg.w
         ctx = self.ctx
         na = plan.anchor.ndims
         big = "0x3fffffff"
+        ctx.floor_div = True
+        self.shifts = []
         for n in plan.nodes:
             nm = self.node_name(n)
             fnm = pg.fn(n.func)
             nd = n.ndims
-            if n.func is plan.anchor:
-                for d in range(nd):
-                    w("const int r_%s_lo%d = pm_imax(a_lo%d, d_%s_lo%d), "
-                      "r_%s_hi%d = pm_imin(a_hi%d, d_%s_hi%d);" % (
-                          nm, d, d, fnm, d, nm, d, d, fnm, d))
-                self.effective_bounds(n)
-                continue
+            los = [[] for _ in range(nd)]
+            his = [[] for _ in range(nd)]
             if n.role == 'out':
                 owner = " && ".join("t%d == 0" % kk
                                     for kk in range(na - nd)) or "true"
                 for d in range(nd):
-                    kk = n.owned_map[d]
+                    kk = d if n.func is plan.anchor else n.owned_map[d]
+                    los[d].append("a_lo%d" % kk)
+                    his[d].append("a_hi%d" % kk if self.const_dim(
+                        plan.anchor, kk) else "a_lo%d + %d" % (
+                            kk, plan.tile[kk] - 1))
+                    if n.func is plan.anchor:
+                        continue
                     w("int o_%s_lo%d = (%s) ? pm_imax(a_lo%d, d_%s_lo%d) : "
                       "%s;" % (nm, d, owner, kk, fnm, d, big))
                     w("int o_%s_hi%d = (%s) ? pm_imin(a_hi%d, d_%s_hi%d) : "
                       "-%s;" % (nm, d, owner, kk, fnm, d, big))
-                    w("int r_%s_lo%d = o_%s_lo%d, r_%s_hi%d = o_%s_hi%d;" % (
-                        nm, d, nm, d, nm, d, nm, d))
-            else:
-                for d in range(nd):
-                    w("int r_%s_lo%d = %s, r_%s_hi%d = -%s;" % (nm, d, big,
-                                                                nm, d, big))
+            guarded = []          # uses whose consumer box can be empty
             for m, per_dim in self.distinct_uses(n):
-                mn = self.node_name(m)
-                w.open("if (!(%s))" % self.empty_expr(m, "e"))
+                mb = [self.use_bounds(m, d) for d in range(m.ndims)]
+                can = [d for d in range(m.ndims) if "pm_im" in "".join(mb[d])]
+                per = []
                 for d, fns in enumerate(per_dim):
+                    ls, hs = [], []
                     for fn in fns:
                         if fn.kind == 'mono':
-                            a = ctx.expr(fn.expr, {fn.var: "e_%s_lo%d" % (
-                                mn, fn.cdim)})
-                            b = ctx.expr(fn.expr, {fn.var: "e_%s_hi%d" % (
-                                mn, fn.cdim)})
+                            t = [ctx.unclamped(fn.expr, {fn.var: b})
+                                 for b in mb[fn.cdim]]
+                            if fn.dir < 0:
+                                t.reverse()
                         elif fn.kind == 'const':
-                            a = b = ctx.expr(fn.expr, {})
+                            t = [ctx.expr(fn.expr, {})] * 2
                         else:
-                            a, b = ("d_%s_lo%d" % (fnm, d),
-                                    "d_%s_hi%d" % (fnm, d))
-                        w("{ const int ea = %s, eb = %s; r_%s_lo%d = "
-                          "pm_imin(r_%s_lo%d, pm_imin(ea, eb)); r_%s_hi%d = "
-                          "pm_imax(r_%s_hi%d, pm_imax(ea, eb)); }" % (
-                              a, b, nm, d, nm, d, nm, d, nm, d))
+                            t = ["d_%s_lo%d" % (fnm, d),
+                                 "d_%s_hi%d" % (fnm, d)]
+                        if t[0] not in ls:
+                            ls.append(t[0])
+                        if t[1] not in hs:
+                            hs.append(t[1])
+                    per.append((ls, hs))
+                if can:
+                    guarded.append((" && ".join("%s <= %s" % mb[d]
+                                                for d in can), per))
+                    continue
+                for d, (ls, hs) in enumerate(per):
+                    los[d] += [t for t in ls if t not in los[d]]
+                    his[d] += [t for t in hs if t not in his[d]]
+            moved = n.in_smem and any(
+                not self.const_dim(n.func, d) and not self.meets_domain(n, d)
+                for d in range(nd))
+            cq = "int" if guarded or moved else "const int"
+
+            def clampd(d, lo, hi):
+                if self.const_dim(n.func, d) and n.role not in (
+                        'global', 'inline'):
+                    return ("pm_imax(%s, d_%s_lo%d)" % (lo, fnm, d),
+                            "pm_imin(%s, d_%s_hi%d)" % (hi, fnm, d))
+                return lo, hi
+            for d in range(nd):
+                lo = _fold("pm_imin", los[d], big)
+                hi = _fold("pm_imax", his[d], "-" + big)
+                if not guarded:
+                    lo, hi = clampd(d, lo, hi)
+                w("%s r_%s_lo%d = %s, r_%s_hi%d = %s;" % (cq, nm, d, lo, nm,
+                                                          d, hi))
+            for cond, per in guarded:
+                w.open("if (%s)" % cond)
+                for d, (ls, hs) in enumerate(per):
+                    w("r_%s_lo%d = %s; r_%s_hi%d = %s;" % (
+                        nm, d, _fold("pm_imin", ["r_%s_lo%d" % (nm, d)] + ls,
+                                     big),
+                        nm, d, _fold("pm_imax", ["r_%s_hi%d" % (nm, d)] + hs,
+                                     "-" + big)))
                 w.close()
-            if n.role not in ('global', 'inline'):
-                # footprint-only nodes stay unclamped (used by pm_inside)
+            if guarded:
                 for d in range(nd):
-                    w("r_%s_lo%d = pm_imax(r_%s_lo%d, d_%s_lo%d); r_%s_hi%d ="
-                      " pm_imin(r_%s_hi%d, d_%s_hi%d);" % (
-                          nm, d, nm, d, fnm, d, nm, d, nm, d, fnm, d))
-            self.effective_bounds(n)
-        # Interior tile: every region is its full static box (nothing was
-        # clamped), HBM reads stay in their buffers, and every stage's single
-        # box-shaped Case holds on its whole region, so the stages can be
+                    lo, hi = clampd(d, "r_%s_lo%d" % (nm, d),
+                                    "r_%s_hi%d" % (nm, d))
+                    if self.const_dim(n.func, d):
+                        w("r_%s_lo%d = %s; r_%s_hi%d = %s;" % (
+                            nm, d, lo, nm, d, hi))
+            self.gen_clamp_shift(n)
+        ctx.floor_div = False
+        # Interior tile: every stage's region lies in its domain, its Cases
+        # are decided the same way on the whole region, HBM reads stay in
+        # their buffers and no clamped tap clamps, so the stages are
         # evaluated without conditions, guards or clamped reads.
         conds = []
-        for n in plan.nodes:
+
+        def need(c):
+            if c not in conds:
+                conds.append(c)
+        for f in plan.steps:
+            if not self.fastable(f) or not self.can_be_inside(f):
+                continue
+            n = plan.node_of[f]
             nm = self.node_name(n)
-            fnm = pg.fn(n.func)
-            if n.role == 'global':
-                for d in range(n.ndims):
-                    if all(fns[d].kind != 'full' for _, fns in n.uses):
-                        conds.append("r_%s_lo%d >= d_%s_lo%d && r_%s_hi%d <= "
-                                     "d_%s_hi%d" % (nm, d, fnm, d, nm, d,
-                                                    fnm, d))
-                continue
-            if n.role == 'inline':
-                continue
+            fnm = pg.fn(f)
+            pre = ""
+            if n.role == 'out' and n.func is not plan.anchor and \
+                    not n.also_smem and n.ndims < na:
+                pre = "o_%s_lo0 > o_%s_hi0 || " % (nm, nm)
             for d, e in enumerate(self.loop_ext(n)):
-                conds.append("r_%s_hi%d - r_%s_lo%d + 1 == %d" % (nm, d, nm,
-                                                                  d, e))
-        inside = self.inside_conds()
-        self.has_inside = inside is not None and \
-            'no_inside' not in pg.p.options
+                if self.const_dim(f, d):
+                    c = "r_%s_hi%d - r_%s_lo%d + 1 == %d" % (nm, d, nm, d, e)
+                else:
+                    c = "r_%s_lo%d >= d_%s_lo%d && r_%s_hi%d <= d_%s_hi%d" % (
+                        nm, d, fnm, d, nm, d, fnm, d)
+                need("(%s(%s))" % (pre, c) if pre else c)
+            for c in self.main_conds(f, n):
+                need("(%s%s)" % (pre, c) if pre else c)
+            for n2, fns in self.inline_uses(n):
+                nm2 = self.node_name(n2)
+                fn2 = pg.fn(n2.func)
+                if n2.role == 'inline':
+                    for c in self.main_conds(n2.func, n2):
+                        need(c)
+                elif n2.role == 'global':
+                    for d in range(n2.ndims):
+                        if all(fs[d].kind != 'full' for _, fs in n2.uses):
+                            need("r_%s_lo%d >= d_%s_lo%d && r_%s_hi%d <= "
+                                 "d_%s_hi%d" % (nm2, d, fn2, d, nm2, d, fn2,
+                                                d))
+        self.has_inside = 'no_inside' not in pg.p.options and any(
+            self.fastable(f) for f in plan.steps)
         # clamped indices (min/max against bounds free of loop variables)
         # that do not clamp at either end of their consumer's region do
         # not clamp anywhere in it (the clamp is monotone in a monotone
@@ -2232,66 +2463,364 @@ class StencilGen(object):
                                     unclamp.append(c)
         self.fold_ok = bool(unclamp)
         if self.has_inside:
-            # the clamp checks come last: && evaluates them only on tiles
-            # whose regions are full (no overflow on empty regions)
-            w("const bool pm_inside = %s;" % (
-                " && ".join(conds + inside + unclamp) or "true"))
+            w("const bool pm_inside = %s;" % (" && ".join(
+                conds + ["%s == 0" % t for t in self.shifts] + unclamp) or
+                "false"))
+            w("(void)pm_inside;")
 
-    def effective_bounds(self, n):
-        """Bounds of the points of a node that read their producers: the
-        region intersected with the node's Case box."""
+    def gen_clamp_shift(self, n):
+        """A buffer read through clamped taps holds the clamped positions
+        too as long as its region meets the domain.  Where that is not
+        certain (a single tap ``f(max(x - 5, 0))`` over a 4-point tile),
+        the region is moved until it does; such a tile runs on the guarded
+        path only (its origins have other residues)."""
+        if not n.in_smem:
+            return
+        w = self.pg.w
+        ctx = self.ctx
+        nm = self.node_name(n)
+        for d in range(n.ndims):
+            if self.const_dim(n.func, d) or self.meets_domain(n, d):
+                continue
+            lo, hi = [], []
+            for m, per_dim in self.distinct_uses(n):
+                for fn in per_dim[d]:
+                    if fn.kind == 'mono' and _has_clamp(fn.expr):
+                        mb = self.use_bounds(m, fn.cdim)
+                        t = [ctx.expr(fn.expr, {fn.var: b}) for b in mb]
+                        lo.append(t[0 if fn.dir > 0 else 1])
+                        hi.append(t[1 if fn.dir > 0 else 0])
+            t = "pm_sh_%s_%d" % (nm, d)
+            w("const int %s = pm_imax(0, %s - r_%s_hi%d) + pm_imin(0, %s - "
+              "r_%s_lo%d);" % (t, _fold("pm_imax", hi, "0"), nm, d,
+                               _fold("pm_imin", lo, "0"), nm, d))
+            w("r_%s_lo%d += %s; r_%s_hi%d += %s;" % (nm, d, t, nm, d, t))
+            self.shifts.append(t)
+
+    def meets_domain(self, n, d):
+        """Whether the taps of every consumer point include, along
+        dimension ``d``, one that no clamp moves up and one that no clamp
+        moves down (evaluated at both ends of the consumer's domain over a
+        range of parameter values)."""
+        key = (n, d)
+        memo = self.__dict__.setdefault('_meets', {})
+        if key not in memo:
+            memo[key] = self._meets_domain(n, d)
+        return memo[key]
+
+    def _meets_domain(self, n, d):
+        env0 = self.pg.p.int_env()
+        envs = [env0] + [dict((k, t) for k in env0) for t in range(1, 65)]
+        for m, per_dim in self.distinct_uses(n):
+            fns = [fn for fn in per_dim[d]
+                   if fn.kind == 'mono' and _has_clamp(fn.expr)]
+            for cdim in set(fn.cdim for fn in fns):
+                dom = m.func.domain[cdim]
+                for env in envs:
+                    try:
+                        ends = [eval_int(dom.lowerBound, env),
+                                eval_int(dom.upperBound, env)]
+                        if ends[0] > ends[1]:
+                            continue
+                        for x in ends:
+                            diff = []
+                            for fn in fns:
+                                if fn.cdim != cdim:
+                                    continue
+                                e2 = dict(env)
+                                e2[fn.var] = x
+                                diff.append(
+                                    eval_int(fn.expr, e2) -
+                                    eval_int(_strip_clamps(fn.expr), e2))
+                            if min(diff) > 0 or max(diff) < 0:
+                                return False
+                    except EvalError:
+                        return False
+        return True
+
+    def main_part(self, f):
+        """The (box, expression) of a piecewise definition that holds on
+        most of the domain: a box-shaped Case with at least three quarters
+        of it at the parameter estimates, disjoint from every later Case
+        (a later one takes precedence).  Border cases such as a grid's
+        ghost ring leave one.  None when there is none (the rows of a
+        per-channel definition)."""
+        memo = self.pg.__dict__.setdefault('_main_parts', {})
+        if id(f) not in memo:
+            memo[id(f)] = self._main_part(f)
+        return memo[id(f)]
+
+    def _main_part(self, f):
+        parts = body_parts(f)
+        boxes = part_boxes(f)
+        if parts[0][0] is None and len(parts) == 1:
+            return None
+        if len(boxes) != len(parts) or not all(b[0].exact for b in boxes):
+            return None
+        if len(parts) == 1:
+            return boxes[0][0], parts[0][1]
+        env = self.pg.p.int_env()
+
+        def volume(lo, hi):
+            v = 1
+            for ls, hs in zip(lo, hi):
+                v *= max(0, min(eval_int(e, env) for e in hs) -
+                         max(eval_int(e, env) for e in ls) + 1)
+            return v
+        whole = volume([[d.lowerBound] for d in f.domain],
+                       [[d.upperBound] for d in f.domain])
+        for i, (b, _, expr, _) in enumerate(boxes):
+            try:
+                v = volume([b.lo[x] for x in f.variables],
+                           [b.hi[x] for x in f.variables])
+            except EvalError:
+                return None
+            if 4 * v < 3 * whole:
+                continue
+            if all(_boxes_disjoint(b, o[0], f.variables)
+                   for o in boxes[i + 1:]):
+                return b, expr
+        return None
+
+    def cases_ok(self, f):
+        """Whether ``f`` can be evaluated without conditions where its main
+        part holds, or by a branch chain over exact boxes."""
+        parts = body_parts(f)
+        if len(parts) == 1 and parts[0][0] is None:
+            return True
+        if self.main_part(f) is not None:
+            return True
+        boxes = part_boxes(f)
+        return len(parts) > 1 and len(boxes) == len(parts) and \
+            all(b[0].exact for b in boxes)
+
+    def inline_uses(self, n):
+        """(node, [IndexFn lists per dimension]) of every producer that
+        the points of step node ``n`` read or evaluate."""
+        out = []
+        for n2 in self.plan.nodes:
+            for m, per_dim in self.distinct_uses(n2):
+                if m is n:
+                    out.append((n2, per_dim))
+        return out
+
+    def fastable(self, f):
+        """Whether step ``f`` has an unconditional form (see cases_ok):
+        its own Cases and those of every stage it evaluates in
+        registers."""
+        memo = self.__dict__.setdefault('_fastable', {})
+        if f not in memo:
+            n = self.plan.node_of[f]
+            memo[f] = 'guarded' not in self.pg.p.options and \
+                self.cases_ok(f) and all(
+                    n2.role != 'inline' or self.cases_ok(n2.func)
+                    for n2, _ in self.inline_uses(n))
+        return memo[f]
+
+    def cover(self, n):
+        """{dimension: (offset, count)}: the points of a shared-memory
+        stage along its dimensions of constant extent that its one Case
+        covers, when that is a proper part of the region and the same on
+        every tile (the bilateral grid's blurs are read at every intensity
+        bin but defined on the inner ones).  The others are 0: they are
+        filled once per tile, and the stage's loops leave them out."""
+        memo = self.__dict__.setdefault('_cover', {})
+        if n.func in memo:
+            return memo[n.func]
+        out = {}
+        mp = self.main_part(n.func)
+        if n.role == 'smem' and mp is not None and \
+                len(body_parts(n.func)) == 1:
+            for d, (lo, hi) in n.const_bounds.items():
+                v = n.func.variables[d]
+                los = [_const_int(e) for e in mp[0].lo[v]]
+                his = [_const_int(e) for e in mp[0].hi[v]]
+                if None in los or None in his or np.any(lo != lo.flat[0]) \
+                        or np.any(hi != hi.flat[0]):
+                    continue
+                a, b = int(lo.flat[0]), int(hi.flat[0])
+                c, e = max([a] + los), min([b] + his)
+                if c <= e and (c, e) != (a, b):
+                    out[d] = (c - a, e - c + 1)
+        memo[n.func] = out
+        return out
+
+    def gen_zero_fill(self, f, n, ext):
+        """Zeros at the region's points outside the covered part of its
+        dimensions of constant extent (see cover)."""
         w = self.pg.w
         nm = self.node_name(n)
-        cb = getattr(n, 'case_box', None)
-        for d in range(n.ndims):
-            lo = "r_%s_lo%d" % (nm, d)
-            hi = "r_%s_hi%d" % (nm, d)
-            if cb:
-                for e in cb[d][0]:
-                    lo = "pm_imax(%s, %s)" % (lo, self.ctx.expr(e, {}))
-                for e in cb[d][1]:
-                    hi = "pm_imin(%s, %s)" % (hi, self.ctx.expr(e, {}))
-            w("const int e_%s_lo%d = %s, e_%s_hi%d = %s;" % (nm, d, lo, nm,
-                                                             d, hi))
+        cov = self.cover(n)
+        tot = 1
+        for e in ext:
+            tot *= e
+        w.open("for (int i = threadIdx.x; i < %d; i += %d)" % (
+            tot, self.plan.threads))
+        self.decompose("i", ext, "j")
+        w("if (%s) sm_%s[%s] = 0;" % (
+            " || ".join("j%d < %d || j%d >= %d" % (d, o, d, o + c)
+                        for d, (o, c) in sorted(cov.items())), nm,
+            " + ".join("j%d * %d" % (d, st)
+                       for d, st in enumerate(n._sm_strides))))
+        w.close()
 
-    def inside_conds(self):
-        """Tile-level conditions under which every stage's Case holds on the
-        stage's whole region; None when some stage is piecewise or its
-        condition is not a box."""
-        pg = self.pg
-        plan = self.plan
+    def can_be_inside(self, f):
+        """Whether some tile's whole region of step ``f`` lies in its main
+        part, as far as the dimensions of constant extent tell: the
+        bilateral grid's last blur is read at every intensity bin but
+        defined on the inner ones only, so it never does."""
+        n = self.plan.node_of[f]
+        mp = self.main_part(f)
+        for d, (lo, hi) in n.const_bounds.items():
+            ok = hi - lo + 1 == self.loop_ext(n)[d]
+            if mp is not None and d not in self.cover(n):
+                for e in mp[0].lo[f.variables[d]]:
+                    if _const_int(e) is not None:
+                        ok = ok & (lo >= _const_int(e))
+                for e in mp[0].hi[f.variables[d]]:
+                    if _const_int(e) is not None:
+                        ok = ok & (hi <= _const_int(e))
+            if not np.any(ok):
+                return False
+        return True
+
+    def main_conds(self, f, n):
+        """Conditions under which ``f``'s main part holds on the whole
+        region of its node."""
         ctx = self.ctx
+        mp = self.main_part(f)
+        if mp is None:
+            return []
+        nm = self.node_name(n)
         out = []
-        for f in plan.funcs:
-            parts = body_parts(f)
-            if len(parts) == 1 and parts[0][0] is None:
+        for d, v in enumerate(f.variables):
+            if n.role == 'smem' and d in self.cover(n):
                 continue
-            if len(parts) != 1:
-                # several box-shaped Cases (e.g. one per channel): evaluated
-                # per point by a branch chain in the interior path
-                boxes = part_boxes(f)
-                if len(boxes) != len(parts) or \
-                        not all(b[0].exact for b in boxes):
-                    return None
-                continue
-            boxes = part_boxes(f)
-            if len(boxes) != 1 or not boxes[0][0].exact:
-                return None
-            n = plan.node_of.get(f)
-            if n is None:
-                continue              # never evaluated in this group
-            box = boxes[0][0]
-            nm = self.node_name(n)
-            for d, v in enumerate(f.variables):
-                for e in box.lo[v]:
-                    c = "r_%s_lo%d >= %s" % (nm, d, ctx.expr(e, {}))
-                    if c not in out:
-                        out.append(c)
-                for e in box.hi[v]:
-                    c = "r_%s_hi%d <= %s" % (nm, d, ctx.expr(e, {}))
-                    if c not in out:
-                        out.append(c)
+            for e in mp[0].lo[v]:
+                out.append("r_%s_lo%d >= %s" % (nm, d, ctx.expr(e, {})))
+            for e in mp[0].hi[v]:
+                out.append("r_%s_hi%d <= %s" % (nm, d, ctx.expr(e, {})))
         return out
+
+    def solve(self, e, var, t, ge):
+        """Bound on ``var`` that makes the monotone index ``e`` (its clamps
+        dropped) >= ``t`` (``ge``) or <= ``t``: ('lo' | 'hi', C text), or
+        None when the form is not handled.  A quotient is taken rounded
+        down, which for the lower bound is the stricter reading."""
+        ctx = self.ctx
+        arm = _clamp_arm(e)
+        if arm is not None:
+            return self.solve(arm, var, t, ge)
+        if e is var:
+            return ('lo' if ge else 'hi', t)
+        f = affine_form(e)
+        if f is not None:
+            co = dict(f[0])
+            a = co.pop(var, None)
+            if not a or any(not isinstance(k, C.Parameter) for k in co):
+                return None
+            rest = ["%d * %s" % (c, ctx.expr(k, {})) for k, c in co.items()]
+            if f[1]:
+                rest.append(str(f[1]))
+            if rest:
+                t = "(%s - (%s))" % (t, " + ".join(rest))
+            if a < 0:
+                a, t, ge = -a, "(-%s)" % t, not ge
+            if a == 1:
+                return ('lo' if ge else 'hi', t)
+            if ge:
+                return ('lo', "(-pm_floordiv(-%s, %d))" % (t, a))
+            return ('hi', "pm_floordiv(%s, %d)" % (t, a))
+        if not isinstance(e, AbstractBinaryOpNode):
+            return None
+        lv, rv = _has_loop_var(e.left), _has_loop_var(e.right)
+        if e.op in '+-' and lv != rv:
+            free = ctx.expr(e.right if lv else e.left, {})
+            if e.op == '+':
+                return self.solve(e.left if lv else e.right, var,
+                                  "(%s - %s)" % (t, free), ge)
+            if lv:
+                return self.solve(e.left, var, "(%s + %s)" % (t, free), ge)
+            return self.solve(e.right, var, "(%s - %s)" % (free, t), not ge)
+        k = _const_int(e.right) if lv and not rv else None
+        if e.op == '/' and k is not None and k > 0:
+            return self.solve(e.left, var, "(%s * %d)" % (t, k) if ge else
+                              "(%s * %d + %d)" % (t, k, k - 1), ge)
+        return None
+
+    def valid_box(self, f, n):
+        """Bounds of the points of step ``f`` that its unconditional form
+        computes correctly: per dimension ([lower bounds], [upper
+        bounds]) as C text, and uniform conditions without which no point
+        qualifies."""
+        pg = self.pg
+        ctx = self.ctx
+        nd = n.ndims
+        nm = self.node_name(n)
+        fnm = pg.fn(f)
+        lo = [["r_%s_lo%d" % (nm, d), "d_%s_lo%d" % (fnm, d)]
+              for d in range(nd)]
+        hi = [["r_%s_hi%d" % (nm, d), "d_%s_hi%d" % (fnm, d)]
+              for d in range(nd)]
+        flags = []
+
+        def add(d, side, t):
+            lst = (lo if side == 'lo' else hi)[d]
+            if t not in lst:
+                lst.append(t)
+
+        def require(fn, t, ge, dom):
+            """``fn`` >= t or <= t at every point; ``dom``: the bounds of
+            the producer's dimension, for data-dependent indices."""
+            if fn.kind == 'mono':
+                b = self.solve(fn.expr, fn.var, t, ge)
+                if b is not None:
+                    add(fn.cdim, b[0], b[1])
+                    return
+                c = []
+                for end in ("lo", "hi"):
+                    c.append("%s %s %s" % (ctx.unclamped(
+                        fn.expr, {fn.var: "r_%s_%s%d" % (nm, end, fn.cdim)}),
+                        ">=" if ge else "<=", t))
+                c = " && ".join(c)
+            elif fn.kind == 'const':
+                c = "%s %s %s" % (ctx.expr(fn.expr, {}), ">=" if ge else
+                                  "<=", t)
+            else:
+                c = "%s %s %s" % (dom[0] if ge else dom[1], ">=" if ge else
+                                  "<=", t)
+            if c not in flags:
+                flags.append(c)
+
+        mp = self.main_part(f)
+        if mp is not None:
+            for d, v in enumerate(f.variables):
+                for e in mp[0].lo[v]:
+                    add(d, 'lo', ctx.expr(e, {}))
+                for e in mp[0].hi[v]:
+                    add(d, 'hi', ctx.expr(e, {}))
+        for n2, per_dim in self.inline_uses(n):
+            f2 = n2.func
+            fn2 = pg.fn(f2)
+            mp = self.main_part(f2) if n2.role == 'inline' else None
+            for d, fns in enumerate(per_dim):
+                dom = ("d_%s_lo%d" % (fn2, d), "d_%s_hi%d" % (fn2, d))
+                for fn in fns:
+                    if mp is not None:
+                        v = f2.variables[d]
+                        for e in mp[0].lo[v]:
+                            require(fn, ctx.expr(e, {}), True, dom)
+                        for e in mp[0].hi[v]:
+                            require(fn, ctx.expr(e, {}), False, dom)
+                    elif n2.role == 'global' and fn.kind != 'full':
+                        require(fn, dom[0], True, dom)
+                        require(fn, dom[1], False, dom)
+                    if fn.kind == 'mono' and _has_clamp(fn.expr) and \
+                            'no_fold_clamps' not in pg.p.options:
+                        for arm, bound, is_min in _clamps(fn.expr):
+                            c = _ArmFn(fn, arm)
+                            require(c, ctx.expr(bound, {}), not is_min, dom)
+        return lo, hi, flags
 
     def distinct_uses(self, n):
         """Uses of a node grouped by consumer, with per-dimension index
@@ -2480,27 +3009,24 @@ class StencilGen(object):
             if written_flag:
                 w("%s = true;" % written_flag)
             return
-        if self.inside and len(parts) == 1:
-            # the single Case holds on the whole region of this tile
-            e = ctx.expr(parts[0][1], bind)
-            w("%s = (%s)(%s);" % (target, ctype(f.typ), e))
-            if written_flag:
-                w("%s = true;" % written_flag)
-            return
-        if self.fast and not self.inside:
-            # unguarded: every case evaluated, later cases take precedence
-            T = ctype(f.typ)
-            val = "(%s)0" % T
-            cs = []
-            for cond, expr, red in parts:
-                c = ctx.cond(cond, bind) if cond is not None else "true"
-                e = ctx.expr(expr, bind)
-                cs.append(c)
-                val = "(%s ? (%s)(%s) : %s)" % (c, T, e, val)
-            w("%s = %s;" % (target, val))
-            if written_flag:
-                w("%s = %s;" % (written_flag, " || ".join(cs)))
-            return
+        if self.inside:
+            main = self.main_part(f)
+            if main is not None:
+                # the main part holds at every point evaluated here
+                e = ctx.expr(main[1], bind)
+                w("%s = (%s)(%s);" % (target, ctype(f.typ), e))
+                if written_flag:
+                    w("%s = true;" % written_flag)
+                return
+        # conditions that read producers are evaluated before the branch
+        # chain (their reads are statements)
+        texts = {}
+        if any(c is not None and c.has(C.Reference) for c, _, _ in parts):
+            for c, _, _ in parts:
+                if c is not None and _cond_static(c, bind) is None:
+                    t = ctx.temp()
+                    w("const bool %s = %s;" % (t, ctx.cond(c, bind)))
+                    texts[id(c)] = t
         first = True
         for cond, expr, red in reversed(parts):
             known = True if cond is None else _cond_static(cond, bind)
@@ -2519,7 +3045,7 @@ class StencilGen(object):
             if known is True:
                 w.open("else")
             else:
-                c = ctx.cond(cond, bind)
+                c = texts.get(id(cond)) or ctx.cond(cond, bind)
                 w.open("%sif (%s)" % ("" if first else "else ", c))
             e = ctx.expr(expr, bind)
             w("%s = (%s)(%s);" % (target, ctype(f.typ), e))
@@ -2656,16 +3182,30 @@ class StencilGen(object):
             return res
         env = self.pg.p.int_env()
         big = 1 << 20
-        # far interior tiles, 8 consecutive along every anchor dim (a full
-        # period of any residue mod 8 of a region origin whose scale
+        # far tiles, 8 consecutive along every parametric anchor dim (a
+        # full period of any residue mod 8 of a region origin whose scale
         # factors divide the tile sizes; others show up as several values)
-        grids = np.meshgrid(*[np.arange(8, dtype=np.int64)] * na,
-                            indexing='ij')
+        # and the actual ones along dims of constant extent
+        axes = []
+        for k, t in enumerate(plan.tile):
+            dom = plan.anchor.domain[k]
+            if self.const_dim(plan.anchor, k):
+                axes.append(np.arange(eval_int(dom.lowerBound, env),
+                                      eval_int(dom.upperBound, env) + 1, t,
+                                      dtype=np.int64))
+            else:
+                axes.append((glo[k] if glo[k] is not None else 0) +
+                            (big + np.arange(8, dtype=np.int64)) * t)
+        grids = np.meshgrid(*axes, indexing='ij')
         box = []
         for k, t in enumerate(plan.tile):
-            lo = (glo[k] if glo[k] is not None else 0) + \
-                (big + grids[k].ravel()) * t
-            box.append((lo, lo + t - 1))
+            lo = grids[k].ravel()
+            hi = lo + t - 1
+            if self.const_dim(plan.anchor, k):
+                hi = np.minimum(hi, axes[k][0] + eval_int(
+                    plan.anchor.domain[k].upperBound -
+                    plan.anchor.domain[k].lowerBound, env))
+            box.append((lo, hi))
         try:
             reg = infer_regions(plan, box, env, clamp=False)
         except Exception:
@@ -2698,7 +3238,8 @@ class StencilGen(object):
         none is a strided HBM read (decided by generating the loop once
         into a scratch buffer)."""
         pg = self.pg
-        if 'no_vec' in pg.p.options or ext[-1] % 4 or ext[-1] < 16:
+        if 'no_vec' in pg.p.options or ext[-1] % 4 or ext[-1] < 16 or \
+                n.ndims - 1 in self.cover(n):
             return 1
         self.inner_residues()
         if f not in self._loop_res:
@@ -2769,34 +3310,52 @@ class StencilGen(object):
         plan = self.plan
         w = pg.w
         n = plan.node_of[f]
+        nm = self.node_name(n)
         ext = self.loop_ext(n)
         w("// stage %s (%s%s)" % (f.name, n.role,
                                   "+smem" if n.also_smem else ""))
-        w.open("")
-        if 'guarded' in pg.p.options:
-            self.gen_guarded_loop(f, n, ext)
+        if n.role == 'out' and n.func is not plan.anchor and \
+                not n.also_smem and n.ndims < plan.anchor.ndims:
+            # a live-out of fewer dimensions: its first tiles write it
+            w.open("if (!(%s))" % " || ".join(
+                "o_%s_lo%d > o_%s_hi%d" % (nm, d, nm, d)
+                for d in range(n.ndims)))
         else:
-            if self.has_inside:
+            w.open("")
+        if self.has_inside and self.fastable(f):
+            if n.role == 'smem' and self.cover(n):
+                self.gen_zero_fill(f, n, ext)
+                ext = [self.cover(n)[d][1] if d in self.cover(n) else e
+                       for d, e in enumerate(ext)]
+            self.fast_mode(True)
+            self.vec = self.choose_vec(f, n, ext)
+            blk = self.block_shape(n, ext)
+            if self.can_be_inside(f):
                 w.open("if (pm_inside)")
-                self.fast = self.inside = True
-                self.ctx.fold_clamps = self.fold_ok
-                self.vec = self.choose_vec(f, n, ext)
-                self.gen_fast_loop(f, n, ext)
-                self.vec = 1
-                self.ctx.fold_clamps = False
-                self.fast = self.inside = False
+                self.gen_fast_loop(f, n, ext, blk)
                 w.close()
                 w.open("else")
-            # every point of the static box, select-based cases, clamped
-            # reads: valid on any tile
-            self.fast = self.clamp = True
-            self.gen_fast_loop(f, n, ext)
-            self.fast = self.clamp = False
-            if self.has_inside:
-                w.close()
+            else:
+                w.open("")
+            self.fast_mode(False)
+            # border tiles: the blocks that lie where the unconditional
+            # form holds run it, the points outside them one at a time
+            self.gen_fast_box(f, n, ext, blk)
+            self.fast_mode(True)
+            self.gen_fast_loop(f, n, ext, blk, "pm_fbox")
+            self.fast_mode(False)
+            self.vec = 1
+            self.gen_slabs(f, n)
+            w.close()
+        else:
+            self.gen_guarded_loop(f, n, ext)
         w.close()
         if n.in_smem:
             w("__syncthreads();")
+
+    def fast_mode(self, on):
+        self.inside = on
+        self.ctx.fold_clamps = on and self.fold_ok
 
     def _store(self, f, n, qs, val, flag, smem_idx, gidx=None,
                hbm=True):
@@ -2815,9 +3374,6 @@ class StencilGen(object):
             if n.func is not plan.anchor and n.also_smem:
                 own = " && ".join("%s >= o_%s_lo%d && %s <= o_%s_hi%d" % (
                     qs[d], nm, d, qs[d], nm, d) for d in range(nd))
-            elif self.clamp:
-                own = " && ".join("%s >= r_%s_lo%d && %s <= r_%s_hi%d" % (
-                    qs[d], nm, d, qs[d], nm, d) for d in range(nd))
             cond = " && ".join(x for x in [own, flag or ""] if x)
             idx = gidx or " + ".join(
                 ["(long long)(%s - d_%s_lo%d) * s_%s_%d" % (qs[d], fnm, d,
@@ -2828,68 +3384,77 @@ class StencilGen(object):
             else:
                 w("b_%s[%s] = %s;" % (fnm, idx, val))
 
-    def gen_guarded_loop(self, f, n, ext):
-        """Border tiles: one point per iteration, guarded by the region."""
+    def gen_point(self, f, n):
+        """One point ``q0..`` of step ``f`` with its conditions evaluated
+        and every read guarded: the form for points near a border."""
         pg = self.pg
-        plan = self.plan
         w = pg.w
         nm = self.node_name(n)
         nd = n.ndims
         comp = pg.p.func_map[f]
-        tot = 1
-        for e in ext:
-            tot *= e
-        w.open("for (int i = threadIdx.x; i < %d; i += %d)" % (
-            tot, plan.threads))
-        self.decompose("i", ext, "j")
-        lv = _loop_vars(nd)
-        for d in range(nd):
-            w("const int q%d = r_%s_lo%d + j%d;" % (d, nm, d, d))
-        w("if (%s) continue;" % " || ".join("q%d > r_%s_hi%d" % (d, nm, d)
-                                           for d in range(nd)))
         ctx = self.ctx
         ctx.push()
-        bind = dict(zip(f.variables, lv))
+        saved_lo = dict(ctx.var_lo)
+        for d, dom in enumerate(f.domain):
+            lo = _const_int(dom.lowerBound)
+            if lo is not None:
+                ctx.var_lo["q%d" % d] = lo     # points lie in the domain
+        self.clamp = True
         w("%s v = 0;" % ctype(f.typ))
         flag = None
         if n.role == 'out' and comp.is_output:
             w("bool wr = false;")
             flag = "wr"
-        self.emit_cases(f, bind, "v", flag)
-        sidx = "i"
+        self.emit_cases(f, dict(zip(f.variables, _loop_vars(nd))), "v", flag)
+        sidx = None
         if n.in_smem:
-            sidx = " + ".join("j%d * %d" % (d, st) for d, st in
-                              enumerate(n._sm_strides))
+            sidx = " + ".join("(q%d - r_%s_lo%d) * %d" % (d, nm, d, st)
+                              for d, st in enumerate(n._sm_strides))
         self._store(f, n, ["q%d" % d for d in range(nd)], "v", flag, sidx)
+        self.clamp = False
+        ctx.var_lo = saved_lo
         ctx.pop()
-        w.close()
 
-    def gen_fast_loop(self, f, n, ext):
-        """Interior tiles: each thread computes a block of ``rb`` points
-        along the second-innermost dimension (consecutive threads take
-        consecutive innermost points, so shared-memory accesses stay
-        conflict-free and HBM accesses coalesced); reads shared by the
-        block's points are loaded once."""
+    def gen_guarded_loop(self, f, n, ext):
+        """One point per iteration over the static box, guarded by the
+        region and the domain: steps without an unconditional form."""
         pg = self.pg
-        plan = self.plan
         w = pg.w
         nm = self.node_name(n)
+        fnm = pg.fn(f)
         nd = n.ndims
-        comp = pg.p.func_map[f]
+        tot = 1
+        for e in ext:
+            tot *= e
+        w.open("for (int i = threadIdx.x; i < %d; i += %d)" % (
+            tot, self.plan.threads))
+        self.decompose("i", ext, "j")
+        for d in range(nd):
+            w("const int q%d = r_%s_lo%d + j%d;" % (d, nm, d, d))
+        w("if (%s) continue;" % " || ".join(
+            "q%d > r_%s_hi%d || q%d < d_%s_lo%d || q%d > d_%s_hi%d" % (
+                d, nm, d, d, fnm, d, d, fnm, d) for d in range(nd)))
+        self.gen_point(f, n)
+        w.close()
+
+    def block_shape(self, n, ext):
+        """(K, cb): rows along the second-innermost dimension and channels
+        along a small outermost one that a thread computes at once (with
+        ``self.vec`` points along the innermost)."""
+        pg = self.pg
+        nd = n.ndims
         rb_max = int(_opt(pg.p, 'rblock', 4))
-        inner = ext[-1]
+        K = 1
         if nd >= 2:
             outer = ext[-2]
             # block height: fewest rows loaded (block + a 2-row halo) per
             # row computed; a last partial block is shifted back to end at
             # the last row (its overlap is recomputed, same values)
-            K, best = 1, None
+            best = None
             for k in range(min(rb_max, outer), 0, -1):
                 cost = -(-outer // k) * (k + 2)
                 if best is None or cost < best:
                     K, best = k, cost
-        else:
-            outer, K = 1, 1
         # a small outermost dimension (channels) is computed by the same
         # thread, so that reads and index arithmetic shared by the channels
         # of a point are done once
@@ -2898,12 +3463,115 @@ class StencilGen(object):
             cb = ext[0]
             while K > 1 and K * cb > 16:
                 K -= 1
-        V = self.vec if (self.inside and nd >= 2) else 1
+        V = self.vec if nd >= 2 else 1
         if V > 1:
             # 4 consecutive inner points per thread: shared-memory reads of
             # a row become 16-byte vector loads
             while K > 1 and K * cb * V > 16:
                 K -= 1
+        return K, cb
+
+    def gen_fast_box(self, f, n, ext, blk):
+        """``f_lo/f_hi``: the box of the whole blocks inside the step's
+        valid box (all blocks start at multiples of the block size from
+        the region's origin, except a last one that is shifted back to end
+        at the region's end); empty when no block qualifies."""
+        w = self.pg.w
+        nm = self.node_name(n)
+        nd = n.ndims
+        lo, hi, flags = self.valid_box(f, n)
+        K, cb = blk
+        V = self.vec if nd >= 2 else 1
+        flags += ["%s == 0" % t for t in self.shifts]
+        for d in range(nd):
+            w("const int v_lo%d = %s, v_hi%d = %s;" % (
+                d, _fold("pm_imax", lo[d], ""), d,
+                _fold("pm_imin", hi[d], "")))
+            org = "r_%s_lo%d" % (nm, d)
+            if d in self.cover(n) and self.cover(n)[d][0]:
+                org = "(%s + %d)" % (org, self.cover(n)[d][0])
+            B = V if d == nd - 1 else K if d == nd - 2 else \
+                cb if d == 0 else 1
+            if B == 1:
+                w("int f_lo%d = v_lo%d, f_hi%d = v_hi%d;" % ((d,) * 4))
+                continue
+            w("int f_lo%d = %s + (v_lo%d - %s + %d) / %d * %d;" % (
+                d, org, d, org, B - 1, B, B))
+            w("int f_hi%d = %s + pm_floordiv(v_hi%d + 1 - %s, %d) * %d - 1;"
+              % (d, org, d, org, B, B))
+            if ext[d] % B:
+                w("if (v_hi%d >= %s + %d) f_hi%d = %s + %d;" % (
+                    d, org, ext[d] - 1, d, org, ext[d] - 1))
+                w("if (f_lo%d > %s + %d) f_hi%d = f_lo%d - 1;" % (
+                    d, org, ext[d] - B, d, d))
+        w("const bool pm_fbox = %s;" % " && ".join(
+            ["f_lo%d <= f_hi%d" % (d, d) for d in range(nd)] +
+            ["(%s)" % c for c in flags]))
+
+    def gen_slabs(self, f, n):
+        """The points of the step's region (inside its domain) outside the
+        box ``f_lo..f_hi``: per dimension the slab below and the slab
+        above it, each spread over all threads."""
+        w = self.pg.w
+        nm = self.node_name(n)
+        fnm = self.pg.fn(f)
+        nd = n.ndims
+        for d in range(nd):
+            if n.role == 'smem' and d in self.cover(n):
+                # zero outside the covered part, which is filled already
+                w("const int s_lo%d = v_lo%d, s_hi%d = v_hi%d;" % ((d,) * 4))
+                continue
+            w("const int s_lo%d = pm_imax(r_%s_lo%d, d_%s_lo%d), s_hi%d = "
+              "pm_imin(r_%s_hi%d, d_%s_hi%d);" % (d, nm, d, fnm, d, d, nm, d,
+                                                  fnm, d))
+        # no block qualifies: everything is the slab below dimension 0
+        w("if (!pm_fbox) { f_lo0 = s_hi0 + 1; f_hi0 = s_hi0; }")
+        w("#pragma unroll 1")
+        w.open("for (int sl = 0; sl < %d; ++sl)" % (2 * nd))
+        for d in range(nd):
+            if d < nd - 1:
+                w("int l%d = sl < %d ? s_lo%d : f_lo%d, h%d = sl < %d ? "
+                  "s_hi%d : f_hi%d;" % (d, 2 * d + 2, d, d, d, 2 * d + 2, d,
+                                        d))
+            else:
+                w("int l%d = s_lo%d, h%d = s_hi%d;" % (d, d, d, d))
+            w("if (sl == %d) h%d = f_lo%d - 1;" % (2 * d, d, d))
+            w("if (sl == %d) l%d = f_hi%d + 1;" % (2 * d + 1, d, d))
+        w("if (%s) continue;" % " || ".join("l%d > h%d" % (d, d)
+                                            for d in range(nd)))
+        w("const int tot = %s;" % " * ".join("(h%d - l%d + 1)" % (d, d)
+                                             for d in range(nd)))
+        w("#pragma unroll 1")
+        w.open("for (int i = threadIdx.x; i < tot; i += %d)" %
+               self.plan.threads)
+        w("unsigned rr = i;")
+        for d in range(nd - 1, 0, -1):
+            w("const unsigned n%d = h%d - l%d + 1;" % (d, d, d))
+            w("const int q%d = l%d + (int)(rr %% n%d); rr /= n%d;" % (
+                d, d, d, d))
+        w("const int q0 = l0 + (int)rr;")
+        self.gen_point(f, n)
+        w.close()
+        w.close()
+
+    def gen_fast_loop(self, f, n, ext, blk=None, box=None):
+        """The unconditional form: each thread computes a block of ``K``
+        points along the second-innermost dimension (consecutive threads
+        take consecutive innermost points, so shared-memory accesses stay
+        conflict-free and HBM accesses coalesced); reads shared by the
+        block's points are loaded once.  ``box``: only the blocks inside
+        f_lo..f_hi, when the named flag says that there are any."""
+        pg = self.pg
+        plan = self.plan
+        w = pg.w
+        nm = self.node_name(n)
+        nd = n.ndims
+        comp = pg.p.func_map[f]
+        inner = ext[-1]
+        outer = ext[-2] if nd >= 2 else 1
+        K, cb = blk or self.block_shape(n, ext)
+        V = self.vec if nd >= 2 else 1
+        if V > 1:
             self.vec_var = "qb%d" % (nd - 1)
             self.vec_res = self._loop_res[f]
         nblk = -(-outer // K)
@@ -2916,8 +3584,8 @@ class StencilGen(object):
         for e in reversed(ext):
             strides.insert(0, st)
             st *= e
-        w.open("for (int it = threadIdx.x; it < %d; it += %d)" % (
-            total, plan.threads))
+        w.open("%sfor (int it = threadIdx.x; it < %d; it += %d)" % (
+            "if (%s) " % box if box else "", total, plan.threads))
         if V > 1:
             w("const int ji = (it %% %d) * %d; int rr = it / %d;" % (
                 inner // V, V, inner // V))
@@ -2944,7 +3612,17 @@ class StencilGen(object):
                 j = "jo"
             else:
                 j = "j%d" % d
-            w("const int qb%d = r_%s_lo%d + %s;" % (d, nm, d, j))
+            off = self.cover(n)[d][0] if d in self.cover(n) else 0
+            w("const int qb%d = r_%s_lo%d + %s%s;" % (
+                d, nm, d, "%d + " % off if off else "", j))
+        if box:
+            w("if (%s) continue;" % " || ".join(
+                "qb%d < f_lo%d || qb%d > f_hi%d" % (
+                    d, d, d, d) if B == 1 else
+                "qb%d < f_lo%d || qb%d + %d > f_hi%d" % (d, d, d, B - 1, d)
+                for d, B in enumerate(
+                    [V if d == nd - 1 else K if d == nd - 2 else
+                     cb if d == 0 else 1 for d in range(nd)])))
         if n.in_smem:
             strides = list(n._sm_strides)     # rows may be padded
         w("const int ib = %s;" % " + ".join(
@@ -2970,7 +3648,7 @@ class StencilGen(object):
             self.inner_residues()
             lres = self._lo_res.get(f) or [None] * nd
             for d in range(nd):
-                if lres[d] is None:
+                if lres[d] is None or d in self.cover(n):
                     continue
                 if d == nd - 1:
                     m = math.gcd(V, 8) if V > 1 else 1
@@ -3090,6 +3768,8 @@ class StencilGen(object):
             w("D.b_%s = (%s%s*)(%s);" % (
                 pg.fn(f), "" if any(f is n.func for n in self.outs)
                 else "const ", ctype(f.typ), pg.buf_expr(f)))
+        for t, h, e in self.hoisted.values():
+            w("D.%s = (%s)(%s);" % (h, t, ctx.expr(e, {})))
         # grid: union of the out nodes' domains along the anchor dims
         for kk in range(na):
             w("long long glo%d = 0x3fffffff, ghi%d = -0x3fffffff;" % (kk, kk))

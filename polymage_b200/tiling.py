@@ -696,8 +696,8 @@ def case_box(func):
 
 def case_restricted(node, region, env, constant_only=False):
     """A node's region intersected with its Case box.  With
-    ``constant_only`` (static-extent simulation at far tile origins) only
-    bounds that do not depend on parameters are applied."""
+    ``constant_only`` (regions without borders) only the constant bounds
+    of dimensions of constant extent are applied."""
     lo, hi = region
     cb = getattr(node, 'case_box', None)
     if not cb:
@@ -706,6 +706,8 @@ def case_restricted(node, region, env, constant_only=False):
     hi = list(hi)
     env2 = dict((k, v * 3 + 17) for k, v in env.items())
     for d, (los, his) in enumerate(cb):
+        if constant_only and _const_extent(node.func.domain[d], env) is None:
+            continue
         for e in los:
             v = try_eval_int(e, env)
             if v is None or (constant_only and try_eval_int(e, env2) != v):
@@ -758,6 +760,10 @@ def infer_regions(plan, anchor_box, env, clamp=True, tile_first=None):
         if n.role == 'out' and n.func is not plan.anchor and clamp:
             lo = [np.maximum(l, dom[d][0]) for d, l in enumerate(lo)]
             hi = [np.minimum(h, dom[d][1]) for d, h in enumerate(hi)]
+        # unclamped, the image is taken to have no borders: only the
+        # dimensions of constant extent keep theirs
+        fixed = [clamp or _const_extent(q, env) is not None
+                 for q in n.func.domain]
         for m, fns in n.uses:
             mlo, mhi = case_restricted(m, regions[m.func], env,
                                        constant_only=not clamp)
@@ -777,9 +783,11 @@ def infer_regions(plan, anchor_box, env, clamp=True, tile_first=None):
                     a, b = dom[d]
                 lo[d] = np.where(nonempty, np.minimum(lo[d], a), lo[d])
                 hi[d] = np.where(nonempty, np.maximum(hi[d], b), hi[d])
-        if clamp:
-            lo = [np.maximum(l, dom[d][0]) for d, l in enumerate(lo)]
-            hi = [np.minimum(h, dom[d][1]) for d, h in enumerate(hi)]
+        if clamp or n.role not in ('global', 'inline'):
+            lo = [np.maximum(l, dom[d][0]) if fixed[d] else l
+                  for d, l in enumerate(lo)]
+            hi = [np.minimum(h, dom[d][1]) if fixed[d] else h
+                  for d, h in enumerate(hi)]
         regions[n.func] = (lo, hi)
     return regions
 
@@ -876,6 +884,13 @@ def _static_extents(plan, env):
                     ext = max(min(int(ext), dext), 1)
                 e.append(int(max(ext, 1)))
             cur[n.func] = e
+            # the region's bounds, over the simulated tiles, along the
+            # dimensions of constant extent (the same on every tile of
+            # the grid, whatever the image size)
+            n.const_bounds = dict(
+                (d, (np.asarray(lo[d]), np.asarray(hi[d])))
+                for d in range(n.ndims)
+                if _const_extent(n.func.domain[d], env) is not None)
         exts.append(cur)
     for n in plan.nodes:
         a, b = exts[0][n.func], exts[1][n.func]
