@@ -3093,19 +3093,35 @@ class StencilGen(object):
 
     def gen_coop_loads(self):
         """Cooperative loads of the staged inputs that have no tensor map
-        (unaligned buffers), into the current tile's copy."""
+        (a base or a row pitch that is not a multiple of 16 bytes), into
+        the current tile's copy.
+
+        4- and 8-byte elements are copied by ``cp.async`` (no register
+        round trip; the zero-fill form outside the array), a group of
+        lanes per row so that the row's index arithmetic and its bounds
+        tests are done once per row and the copies of a warp are
+        contiguous.  Unsharp 3x1079x1917 (rows of 7684 bytes, 68 x 136
+        floats a tile): 21.0 us, against 27.7 us with one element a
+        thread and iteration.  Narrower elements (cp.async moves 4 bytes
+        at least) keep that form."""
         pg = self.pg
         plan = self.plan
         w = pg.w
+        self.async_loads = False
         for n in self.stage_nodes:
             nm = self.node_name(n)
             fnm = pg.fn(n.func)
             nd = n.ndims
             ext = n._sm_ext
+            es = n.func.typ.size()
             tot = 1
             for e in ext:
                 tot *= e
             w.open("if (!D.tma_%s && !(%s))" % (nm, self.empty_expr(n)))
+            if es in (4, 8) and nd >= 2:
+                self.gen_row_copies(n, nm, fnm, ext, es)
+                w.close()
+                continue
             w.open("for (int i = threadIdx.x; i < %d; i += %d)" % (
                 tot, plan.threads))
             self.decompose("i", ext, "j")
@@ -3125,6 +3141,55 @@ class StencilGen(object):
                 ctype(n.func.typ)))
             w.close()
             w.close()
+        if self.async_loads:
+            w("if (!PM_CH) pm_cp_async_wait();")
+
+    def gen_row_copies(self, n, nm, fnm, ext, es):
+        """cp.async copies of a staged input, ``lanes`` threads a row."""
+        w = self.pg.w
+        plan = self.plan
+        nd = n.ndims
+        inner = ext[-1]
+        # lanes a row: as many as possible (contiguous copies of a warp)
+        # that idle at most a fifth of the lanes over a row
+        best = min(-(-inner // k) * k for k in (32, 16, 8))
+        lanes = max(k for k in (32, 16, 8)
+                    if -(-inner // k) * k <= 1.2 * best)
+        rows = 1
+        for e in ext[:-1]:
+            rows *= e
+        self.async_loads = True
+        w("const int j%d = threadIdx.x %% %d;" % (nd - 1, lanes))
+        w.open("for (int i = threadIdx.x / %d; i < %d; i += %d)" % (
+            lanes, rows, plan.threads // lanes))
+        if nd == 2:
+            w("const int j0 = i;")
+        else:
+            self.decompose("i", ext[:-1], "j")
+        inb, coords = [], []
+        for d in range(nd - 1):
+            w("const int c%d = r_%s_lo%d - d_%s_lo%d + j%d;" % (d, nm, d, fnm,
+                                                               d, d))
+            inb.append("c%d >= 0 && c%d <= d_%s_hi%d - d_%s_lo%d" % (
+                d, d, fnm, d, fnm, d))
+            coords.append("(long long)c%d * s_%s_%d" % (d, fnm, d))
+        # columns [first, last) of the buffer's row lie in the array (none
+        # when the row does not)
+        w("const bool in_row = %s;" % " && ".join(inb))
+        w("const %s* src = b_%s + (in_row ? %s : 0) + so_%s_%d;" % (
+            ctype(n.func.typ), fnm, " + ".join(coords), nm, nd - 1))
+        w("const int first = in_row ? -so_%s_%d : %d;" % (nm, nd - 1, inner))
+        w("const int last = in_row ? d_%s_hi%d - d_%s_lo%d + 1 - so_%s_%d : "
+          "0;" % (fnm, nd - 1, fnm, nd - 1, nm, nd - 1))
+        w("#pragma unroll")
+        w.open("for (int k = 0; k < %d; k += %d)" % (inner, lanes))
+        w("const int j = j%d + k;" % (nd - 1))
+        w("const bool ok = j >= first && j < last;")
+        cond = "" if inner % lanes == 0 else "if (j < %d) " % inner
+        w("%spm_copy<PM_CH>(&sm_%s[i * %d + j], ok ? src + j : b_%s, ok);" %
+          (cond, nm, inner, fnm))
+        w.close()
+        w.close()
 
     def gen_wait(self, bar, bit, other):
         """Wait for the current tile's TMA loads on ``bar`` (phase bit

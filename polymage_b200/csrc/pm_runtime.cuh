@@ -101,6 +101,26 @@ __device__ __forceinline__ T pm_ld(const T* p) {
   else return __ldg(p);
 }
 
+// Copy of one 4- or 8-byte element to shared memory, zero when `ok` is
+// false (`src` must be a readable address all the same): asynchronous, to be
+// waited for with pm_cp_async_wait, in a standalone launch.  At these sizes
+// cp.async allocates in L1, so a body inside a chain kernel, which reads
+// what other CTAs of its launch wrote, copies through a register past L1.
+template <bool CH, typename T>
+__device__ __forceinline__ void pm_copy(T* dst, const T* src, bool ok) {
+  if constexpr (CH) {
+    *dst = ok ? __ldcg(src) : (T)0;
+  } else {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(
+                     pm_smem_addr(dst)),
+                 "l"(src), "n"(sizeof(T)), "r"(ok ? (int)sizeof(T) : 0)
+                 : "memory");
+  }
+}
+__device__ __forceinline__ void pm_cp_async_wait() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
 // Between two phases of a chain kernel: every generic-proxy access of this
 // thread (global stores read by later TMA loads, shared memory that a later
 // group's TMA overwrites) is ordered before later async-proxy accesses.
