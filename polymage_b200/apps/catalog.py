@@ -14,8 +14,7 @@ Harris also runs 128-thread CTAs, on 32x64 tiles (0.0273 vs 0.0291 ms).
 The bilateral grid's construction takes 16x256-pixel tiles (0.0908 vs
 0.1033 ms with 32x256), and its slicing group stages the input pixels by
 TMA although it reads each once (option stage_pointwise: 0.0728 vs 0.0786
-ms; the same option slows the pyramids and the local Laplacian), interpolation 32x64 tiles (0.53 vs 1.69 ms with
-the reference builder's 16x16).  The camera pipe fuses every stage into one
+ms; the same option slows the pyramids and the local Laplacian).  The camera pipe fuses every stage into one
 group (option fuse_all; the greedy grouping leaves six kernels: 0.133 vs
 0.190 ms) and tiles its three output channels whole (option channel_tile:
 a thread computes a pixel's red, green and blue once for all three
@@ -29,21 +28,28 @@ clamped taps unclamped); the bilateral grid is slower with it (0.108 vs
 The widening pipelines' settings are the best of smaller sweeps
 (polymage_b200.apps.measure, same timing): Jacobi 2-D 32x64 tiles with 5
 steps per group (0.133 vs 0.207 ms for 16x64 with 10), Jacobi 3-D and the
-3-D multigrid cycles unfused (group size 1) on 8x16x32 and 8x16x64 tiles
-(0.164 vs 0.356 ms; 3.2 vs 8.6 ms): in 3-D the halo of a fused time step
-grows every face of a tile, so recomputation costs more than the HBM
-round trip it saves.  The Jacobi steps, the 2-D multigrid cycles and NAS MG
-also stage their pointwise-read right-hand sides by TMA (option
-stage_pointwise: Jacobi 2-D 0.116 vs 0.132 ms, 3-D 0.154 vs 0.165 ms,
+3-D multigrid cycles unfused (group size 1; 0.164 vs 0.356 ms and 3.2 vs
+8.6 ms on the larger tiles of that sweep): in 3-D the halo of a fused time
+step grows every face of a tile, so recomputation costs more than the HBM
+round trip it saves.  Their tiles are small, 4x16x32 and 4x8x32 points in
+CTAs of 128 threads, four to nine of which reside on an SM, so that some
+load while others compute (Jacobi 3-D 128^3 0.117 vs 0.139 ms on 8x16x32
+with 256 threads, V-cycle 255^3 1.37 vs 1.96 ms on 8x16x64 with 256;
+4x8x64 and 8x8x64 lie between, tiles 34 or 66 wide, which cover 2^k + 2
+points without a remainder, behind).  The Jacobi steps, the multigrid cycles
+and NAS MG also stage their pointwise-read right-hand sides by TMA (option
+stage_pointwise: Jacobi 2-D 0.116 vs 0.132 ms, 3-D 0.117 vs 0.138 ms,
 V-cycle 0.073 vs 0.083 ms, W-cycle 0.138 vs 0.155 ms, NAS MG 0.255 vs
-0.264 ms; the 3-D cycles are slower with it).
+0.264 ms, 3-D V-cycle 1.17 vs 1.61 ms).
 A later sweep of the CTA-shape knobs (same timing, one box): the camera
 pipe with 3 resident CTAs asked of ptxas (0.0491 vs 0.0553 ms), the L=4
 pyramid with 4 rows per thread and its tile regions computed by one
 thread (option shared_regions: 0.1735 vs 0.1875 ms; every other pipeline
 is slower with that option), the L=8 pyramid and the local Laplacian with
 4 rows per thread (0.2164 vs 0.2237 ms, 0.1474 vs 0.1496 ms),
-interpolation with 3 resident CTAs (0.3048 vs 0.3138 ms).  Harris sums
+interpolation with its four channels tiled whole (option channel_tile_all:
+the channels share the alpha channel's work) on 16x64 tiles (0.172 vs
+0.299 ms; 0.181 on 32x64, 0.208 on 8x64).  Harris sums
 its 3x3 box sums and Sobel taps as row sums that the rows of a thread's
 block share (option separable: 0.0255 vs 0.0274 ms).  The 2-D multigrid
 cycles take 8x32 tiles: their 255^2 grids give 16x64 tiles too few CTAs
@@ -97,13 +103,14 @@ INTERPOLATE = dict(rows=2048, cols=2048, tile_sizes=(16, 64), group_size=11,
                    options=('channel_tile_all',))
 JACOBI2D = dict(N=2048, T=10, tile_sizes=(32, 64), group_size=5,
                 options=('stage_pointwise',))
-JACOBI3D = dict(N=128, T=10, tile_sizes=(8, 16, 32), group_size=1,
-                options=('stage_pointwise',))
+JACOBI3D = dict(N=128, T=10, tile_sizes=(4, 16, 32), group_size=1,
+                options=('stage_pointwise', 'threads=128'))
 VCYCLE = dict(n=31, L=3, nu1=10, nu2=0, nuc=0, tile_sizes=(8, 32),
               group_size=6, options=('stage_pointwise',))
 WCYCLE = dict(VCYCLE, gamma=2, name="Wcycle")
 VCYCLE3D = dict(n=31, L=3, nu1=10, nu2=0, nuc=0, dims=3,
-                tile_sizes=(8, 16, 64), group_size=1, name="Vcycle3d")
+                tile_sizes=(4, 8, 32), group_size=1, name="Vcycle3d",
+                options=('stage_pointwise', 'threads=128'))
 WCYCLE3D = dict(VCYCLE3D, gamma=2, name="Wcycle3d")
 MG3P = dict(prob_class='W', tile_sizes=(4, 8, 32), group_size=6,
             options=('stage_pointwise',))

@@ -687,6 +687,13 @@ def _linear(e):
     return {str(e): 1}, 0
 
 
+def _at_most(a, b):
+    """Whether integer bound ``a`` provably does not exceed ``b`` (they
+    differ by a constant)."""
+    p, q = _linear(a), _linear(b)
+    return p[0] == q[0] and p[1] <= q[1]
+
+
 def _boxes_disjoint(a, b, variables):
     """Whether two boxes provably have no common point: along some
     variable a lower bound of one exceeds an upper bound of the other by a
@@ -900,6 +907,78 @@ class PipelineGen(object):
                 self.storage_perm(f) is not None:
             return 1
         return 16 // f.typ.size()
+
+    def need_hi(self, f):
+        """Per dimension of a live-out that is no pipeline output, an upper
+        bound (expression) past which no stage reads it, or None for its
+        domain's.  The multigrid restriction is declared over the fine grid
+        but read on the coarse one only: an eighth of the points."""
+        memo = self.__dict__.setdefault('_need_hi', {})
+        if id(f) not in memo:
+            memo[id(f)] = self._find_need_hi(f)
+        return memo[id(f)]
+
+    def _find_need_hi(self, f):
+        none = [None] * len(f.domain)
+        if isinstance(f, (C.Image, C.Reduction)) or \
+                any(f is o for o in self.outputs) or \
+                getattr(f, 'is_const_func', False) or \
+                'oob_zero' in self.p.options:
+            return none
+        env = self.p.int_env()
+        out = list(none)
+        for d, dom in enumerate(f.domain):
+            reads = self._read_ends(f, d)
+            if not reads:
+                continue
+            # the least of the reads' ends that bounds them all
+            tops = []
+            for top in (e for ends in reads for e in ends):
+                if not _at_most(dom.upperBound, top) and \
+                        all(any(_at_most(e, top) for e in ends)
+                            for ends in reads):
+                    try:
+                        tops.append((eval_int(top, env), len(tops), top))
+                    except EvalError:
+                        pass
+            if tops and min(tops)[0] < eval_int(dom.upperBound, env):
+                out[d] = min(tops)[2]
+        return out
+
+    def _read_ends(self, f, d):
+        """For every read of ``f``, upper bounds (expressions) of its index
+        along dimension ``d`` over the points whose Case reads it; None
+        when some read's index cannot be bounded."""
+        from .pipe import body_refs
+        out = []
+        for comp in self.p.comps:
+            g = comp.func
+            if g is f or not any(r.objectRef is f for r in body_refs(g)):
+                continue
+            for box, cond, expr, red in part_boxes(g):
+                refs = [r for r in expr.collect(C.Reference)
+                        if r.objectRef is f]
+                if cond is not None and cond.has(C.Reference) or \
+                        red is not None and any(
+                            a.has(C.Reference) for a in
+                            red.accumulate_ref.arguments):
+                    return None
+                for r in refs:
+                    a = Value.numericToValue(r.arguments[d])
+                    vs = [x for x in a.collect(C.Variable)
+                          if not isinstance(x, C.Parameter)]
+                    if is_data_dependent(a) or len(set(map(id, vs))) > 1:
+                        return None
+                    if not vs:
+                        out.append([a])
+                        continue
+                    way = monotone_dir(a, vs[0])
+                    ends = {1: box.hi, -1: box.lo}.get(way, {}).get(vs[0])
+                    if not ends:
+                        return None
+                    out.append([substitute_vars(a, {vs[0]: e})
+                                for e in ends])
+        return out
 
     def declare_domain(self, w, f, ctx, need_strides):
         n = self.fn(f)
@@ -2424,6 +2503,10 @@ class StencilGen(object):
                     c = "r_%s_lo%d >= d_%s_lo%d && r_%s_hi%d <= d_%s_hi%d" % (
                         nm, d, fnm, d, nm, d, fnm, d)
                 need("(%s(%s))" % (pre, c) if pre else c)
+            for d, e in enumerate(self.needed(n)):
+                if e is not None:
+                    c = "r_%s_hi%d <= %s" % (nm, d, e)
+                    need("(%s%s)" % (pre, c) if pre else c)
             for c in self.main_conds(f, n):
                 need("(%s%s)" % (pre, c) if pre else c)
             for n2, fns in self.inline_uses(n):
@@ -2540,11 +2623,11 @@ class StencilGen(object):
 
     def main_part(self, f):
         """The (box, expression) of a piecewise definition that holds on
-        most of the domain: a box-shaped Case with at least three quarters
-        of it at the parameter estimates, disjoint from every later Case
-        (a later one takes precedence).  Border cases such as a grid's
-        ghost ring leave one.  None when there is none (the rows of a
-        per-channel definition)."""
+        most of the points that any Case covers: a box-shaped Case with at
+        least three quarters of them at the parameter estimates, disjoint
+        from every later Case (a later one takes precedence).  Border cases
+        such as a grid's ghost ring leave one.  None when there is none
+        (the rows of a per-channel definition)."""
         memo = self.pg.__dict__.setdefault('_main_parts', {})
         if id(f) not in memo:
             memo[id(f)] = self._main_part(f)
@@ -2567,15 +2650,14 @@ class StencilGen(object):
                 v *= max(0, min(eval_int(e, env) for e in hs) -
                          max(eval_int(e, env) for e in ls) + 1)
             return v
-        whole = volume([[d.lowerBound] for d in f.domain],
-                       [[d.upperBound] for d in f.domain])
-        for i, (b, _, expr, _) in enumerate(boxes):
-            try:
-                v = volume([b.lo[x] for x in f.variables],
+        try:
+            vols = [volume([b.lo[x] for x in f.variables],
                            [b.hi[x] for x in f.variables])
-            except EvalError:
-                return None
-            if 4 * v < 3 * whole:
+                    for b, _, _, _ in boxes]
+        except EvalError:
+            return None
+        for i, (b, _, expr, _) in enumerate(boxes):
+            if 4 * vols[i] < 3 * sum(vols):
                 continue
             if all(_boxes_disjoint(b, o[0], f.variables)
                    for o in boxes[i + 1:]):
@@ -2702,6 +2784,14 @@ class StencilGen(object):
                 out.append("r_%s_hi%d <= %s" % (nm, d, ctx.expr(e, {})))
         return out
 
+    def needed(self, n):
+        """Per dimension, the C text of a live-out's last needed point
+        (see need_hi), or None."""
+        if n.role != 'out':
+            return [None] * n.ndims
+        return [e if e is None else self.ctx.expr(e, {})
+                for e in self.pg.need_hi(n.func)]
+
     def solve(self, e, var, t, ge):
         """Bound on ``var`` that makes the monotone index ``e`` (its clamps
         dropped) >= ``t`` (``ge``) or <= ``t``: ('lo' | 'hi', C text), or
@@ -2763,6 +2853,9 @@ class StencilGen(object):
         hi = [["r_%s_hi%d" % (nm, d), "d_%s_hi%d" % (fnm, d)]
               for d in range(nd)]
         flags = []
+        for d, e in enumerate(self.needed(n)):
+            if e is not None:
+                hi[d].append(e)
 
         def add(d, side, t):
             lst = (lo if side == 'lo' else hi)[d]
@@ -3498,7 +3591,9 @@ class StencilGen(object):
             w("const int q%d = r_%s_lo%d + j%d;" % (d, nm, d, d))
         w("if (%s) continue;" % " || ".join(
             "q%d > r_%s_hi%d || q%d < d_%s_lo%d || q%d > d_%s_hi%d" % (
-                d, nm, d, d, fnm, d, d, fnm, d) for d in range(nd)))
+                d, nm, d, d, fnm, d, d, fnm, d) for d in range(nd)) +
+          "".join(" || q%d > %s" % (d, e)
+                  for d, e in enumerate(self.needed(n)) if e is not None))
         self.gen_point(f, n)
         w.close()
 
@@ -3586,9 +3681,11 @@ class StencilGen(object):
                 # zero outside the covered part, which is filled already
                 w("const int s_lo%d = v_lo%d, s_hi%d = v_hi%d;" % ((d,) * 4))
                 continue
+            top = "pm_imin(r_%s_hi%d, d_%s_hi%d)" % (nm, d, fnm, d)
+            if self.needed(n)[d] is not None:
+                top = "pm_imin(%s, %s)" % (top, self.needed(n)[d])
             w("const int s_lo%d = pm_imax(r_%s_lo%d, d_%s_lo%d), s_hi%d = "
-              "pm_imin(r_%s_hi%d, d_%s_hi%d);" % (d, nm, d, fnm, d, d, nm, d,
-                                                  fnm, d))
+              "%s;" % (d, nm, d, fnm, d, d, top))
         # no block qualifies: everything is the slab below dimension 0
         w("if (!pm_fbox) { f_lo0 = s_hi0 + 1; f_hi0 = s_hi0; }")
         w("#pragma unroll 1")
@@ -3841,9 +3938,10 @@ class StencilGen(object):
         for n in self.outs:
             for d, dom in enumerate(n.func.domain):
                 kk = n.owned_map[d] if n.func is not anchor else d
+                hi = self.pg.need_hi(n.func)[d]
                 w("glo%d = pm_llmin(glo%d, %s); ghi%d = pm_llmax(ghi%d, %s);"
                   % (kk, kk, ctx.expr(dom.lowerBound, {}), kk, kk,
-                     ctx.expr(dom.upperBound, {})))
+                     ctx.expr(dom.upperBound if hi is None else hi, {})))
         w("long long tot = 1;")
         for kk in range(na):
             w("if (ghi%d < glo%d) { *ntiles = 0; return PM_OK; }" % (kk, kk))
