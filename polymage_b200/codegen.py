@@ -2133,11 +2133,13 @@ class StencilGen(object):
         pre = bool(self.stage_nodes) and 'prefetch' in pg.p.options and \
             getattr(plan, 'stage_delta', 0) > 0
         self.prefetch = pre
-        if 'pdl' in pg.p.options:
-            # option 'pdl': launched with programmatic stream serialization;
-            # nothing earlier kernels wrote is read before this wait
-            w("pm_grid_dep_wait();")
-            w("pm_grid_dep_launch();")
+        # Programmatic dependent launch (see pm_launch_pdl): the next kernel
+        # of the stream may be scheduled as this one's last CTAs run, and a
+        # kernel so started waits before it reads or writes any array.  In a
+        # chain kernel the phases are ordered by its grid barriers.
+        pdl = 'no_pdl' not in pg.p.options
+        if pdl:
+            w("if (!PM_CH) pm_grid_dep_launch();")
         if self.stage_nodes:
             # one mbarrier per copy of the staged inputs, initialized once;
             # each tile that issues TMA loads completes one phase of the
@@ -2161,6 +2163,8 @@ class StencilGen(object):
             w.open("for (int tile = L.first + pm_bid; tile < L.total; )")
             self.gen_tile_setup("tile")
             self.gen_buffers(None)
+            if pdl:
+                w("if (!PM_CH) pm_grid_dep_wait();")
             if self.stage_nodes:
                 self.gen_issue("pm_bar")
                 self.gen_coop_loads()
@@ -2187,6 +2191,8 @@ class StencilGen(object):
         # alternate between two copies; the loads of tile n+1 are issued
         # (thread 0) before tile n is computed.  The next index is drawn
         # from the queue one tile ahead.
+        if pdl:
+            w("if (!PM_CH) pm_grid_dep_wait();")
         w("int pm_buf = 0;          // copy of the staged inputs this tile "
           "reads")
         w("int tile = L.first + pm_bid;")
@@ -4013,10 +4019,11 @@ class StencilGen(object):
             w("const long long res = %s_resident_now();" % k)
             w("if (nt > res) { grid = res; L.stride = 1; }")
             w.close()
-        if 'pdl' in pg.p.options:
-            w("if (pm_launch_pdl(%s, (unsigned)grid, %d, %d, s, L) != "
-              "cudaSuccess) return PM_ERR_CUDA;" % (k, plan.threads,
-                                                   plan.smem_bytes))
+        if 'no_pdl' not in pg.p.options:
+            w("if (pm_launch_pdl(%s, (unsigned)grid, %d, %d, s, L, %s) != "
+              "cudaSuccess) return PM_ERR_CUDA;" % (
+                  k, plan.threads, plan.smem_bytes,
+                  "true" if 'pdl' in pg.p.options else "false"))
         else:
             w("%s<<<(unsigned)grid, %d, %d, s>>>(L);" % (k, plan.threads,
                                                         plan.smem_bytes))

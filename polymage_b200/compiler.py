@@ -33,8 +33,8 @@ as ``"name=value"`` strings or ``(name, value)`` tuples:
 * reductions: ``red_unroll=N``, ``red_spread``, ``no_gather`` (scatter
   form instead of output-stationary);
 * launches: ``streams=N`` (concurrent streams for independent groups, 1
-  for the caller's stream only), ``pdl`` (programmatic stream
-  serialization), ``chain`` / ``('chain', N)`` (consecutive stencil groups
+  for the caller's stream only), ``pdl`` / ``no_pdl`` (programmatic stream
+  serialization also in captured graphs / nowhere), ``chain`` / ``('chain', N)`` (consecutive stencil groups
   of at most N tiles each as phases of one launch, grid barriers between
   dependent phases);
 * switches of single optimisations, for measurement and debugging:
