@@ -11,10 +11,12 @@ shared-memory stage and its barrier (0.087-0.090 vs 0.094 ms for the
 tuned best); CTAs of 128 threads on 64x128 tiles with 16 rows per thread
 keep more, smaller CTAs resident (0.0773 vs 0.0866 ms with 256 threads).
 Harris also runs 128-thread CTAs, on 32x64 tiles (0.0273 vs 0.0291 ms).
-The bilateral grid's construction takes 16x256-pixel tiles (0.0908 vs
-0.1033 ms with 32x256), and its slicing group stages the input pixels by
-TMA although it reads each once (option stage_pointwise: 0.0728 vs 0.0786
-ms; the same option slows the pyramids and the local Laplacian).  The camera pipe fuses every stage into one
+The bilateral grid's construction takes 16x256-pixel tiles (0.0519 ms for
+both kernels, 0.0526 on 8x256 and 0.0534 on 32x256), and its slicing group
+stages the input pixels by TMA although it reads each once (option
+stage_pointwise: 0.0728 vs 0.0786 ms with the construction of that time;
+the same option slows the pyramids and the local Laplacian) and asks for 3
+resident CTAs (0.0480 vs 0.0508 ms).  The camera pipe fuses every stage into one
 group (option fuse_all; the greedy grouping leaves six kernels: 0.133 vs
 0.190 ms) and tiles its three output channels whole (option channel_tile:
 a thread computes a pixel's red, green and blue once for all three
@@ -23,8 +25,8 @@ Harris and both pyramids ask ptxas for 4 resident CTAs per SM
 (``min_blocks=4``: at most 64 registers a thread), also outside the tuned
 space: 0.0290 vs 0.0303 ms, 0.203 vs 0.209 ms and
 0.218 vs 0.227 ms (the 8-level pyramid with its interior tiles reading
-clamped taps unclamped); the bilateral grid is slower with it (0.108 vs
-0.107 ms) and unsharp is bound by shared memory, not registers.
+clamped taps unclamped); unsharp is bound by shared memory, not
+registers.
 The widening pipelines' settings are the best of smaller sweeps
 (polymage_b200.apps.measure, same timing): Jacobi 2-D 32x64 tiles with 5
 steps per group (0.133 vs 0.207 ms for 16x64 with 10), Jacobi 3-D and the
@@ -80,7 +82,7 @@ CAMPIPE = dict(tile_sizes=(32, 128), group_size=12,
                         'min_blocks=3'))
 BILATERAL = dict(tile_sizes=(1, 32, 128), group_size=10,
                  options=(('red_tile', (16, 256)), 'rblock=4',
-                          'stage_pointwise'))
+                          'stage_pointwise', 'min_blocks=3'))
 PYRAMID = dict(tile_sizes=(32, 64), group_size=10,
                options=('rblock=4', 'min_blocks=4', 'shared_regions'))
 # 8 levels, indices clamped at every level's borders (any image size)

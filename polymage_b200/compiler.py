@@ -31,7 +31,8 @@ as ``"name=value"`` strings or ``(name, value)`` tuples:
   dims), ...))`` (an intermediate array's dimensions, outermost to
   innermost in memory);
 * reductions: ``red_unroll=N``, ``red_spread``, ``no_gather`` (scatter
-  form instead of output-stationary);
+  form instead of output-stationary), ``no_cells`` (atomics instead of
+  per-thread bins for sums into grid cells);
 * launches: ``streams=N`` (concurrent streams for independent groups, 1
   for the caller's stream only), ``pdl`` / ``no_pdl`` (programmatic stream
   serialization also in captured graphs / nowhere), ``chain`` / ``('chain', N)`` (consecutive stencil groups
@@ -41,7 +42,8 @@ as ``"name=value"`` strings or ``(name, value)`` tuples:
   ``shared_regions`` (one thread computes a tile's regions and shares
   them through shared memory), ``no_inside`` (every tile on the general
   path), ``guarded`` (one point per iteration), ``no_vec``, ``no_vec2``,
-  ``no_cblock``, ``no_static_res``, ``no_fold_clamps``.
+  ``no_cblock``, ``no_pairs`` (two channels of a shared-memory stage not
+  interleaved), ``no_static_res``, ``no_fold_clamps``.
 """
 
 from .pipe import Pipeline

@@ -170,6 +170,7 @@ class Node(object):
         self.uses = []                # [(consumer Node, [IndexFn])]
         self.ext = None               # static extents per dim
         self.pad_inner = None         # padded innermost extent (stage)
+        self.pairs = False            # two channels interleaved (smem)
         self.smem_off = None
         self.smem_bytes = 0
         self.step = None              # compute step (0: staged inputs)
@@ -277,11 +278,16 @@ class ReductionPlan(object):
         # every part targets the same cell given by plain reduction
         # variables; None otherwise
         self.gather = None
+        # grid-cell form: (points of a cell along each of the two
+        # reduction variables, the target dimension each maps to, bins of
+        # a cell: the other target dimensions' extents), see _cell_map
+        self.cells = None
 
     def describe(self):
-        return ["reduction %s tile %s privatize %s ext %s gather %s" % (
-            self.func.name, self.tile, self.privatize, self.priv_ext,
-            self.gather)]
+        return ["reduction %s tile %s privatize %s ext %s gather %s "
+                "cells %s" % (
+                    self.func.name, self.tile, self.privatize, self.priv_ext,
+                    self.gather, self.cells)]
 
     def features(self):
         return {'nstages': 1, 'tile_inner': self.tile[-1],
@@ -588,7 +594,10 @@ def plan_stencil(pipeline, comps, tile=None):
     _static_extents(plan, env)
     _alignment(plan, env)
     _layout_smem(plan, tight=('tight_stage' in pipeline.options), env=env,
-                 prefetch=('prefetch' in pipeline.options))
+                 prefetch=('prefetch' in pipeline.options),
+                 no_pairs=bool({'no_pairs', 'no_cblock'} &
+                               set(o for o in pipeline.options
+                                   if isinstance(o, str))))
     if plan.smem_bytes > int(_option(pipeline, 'smem_budget', SMEM_BUDGET)):
         raise PlanError("shared memory %d B exceeds budget" %
                         plan.smem_bytes, list(plan.tile))
@@ -953,7 +962,8 @@ def _alignment(plan, env):
                     raise PlanError("inconsistent scaling of %s" % n.name)
 
 
-def _layout_smem(plan, tight=False, env=None, prefetch=False):
+def _layout_smem(plan, tight=False, env=None, prefetch=False,
+                 no_pairs=False):
     """Shared-memory buffers, placed first-fit by lifetime.  A staged
     input's rows carry the slack a TMA box needs when its origin is
     rounded down to 16 bytes; with ``tight`` (option 'tight_stage') an
@@ -975,6 +985,15 @@ def _layout_smem(plan, tight=False, env=None, prefetch=False):
         es = n.func.typ.size()
         ext = list(n.ext)
         n.tight = False
+        # two channels outermost: stored next to each other, so that a
+        # thread that needs both at a point reads and writes them as one
+        # 8-byte word (dims [c][..][z] at strides 1, .., 2).  The bilateral
+        # grid's slicing gathers 8 pairs a pixel from bins that differ
+        # lane by lane instead of 16 words (50.8 vs 52.7 us a call at
+        # 2560x1536; option 'no_pairs' keeps the planes apart)
+        n.pairs = n.role == 'smem' and es == 4 and n.ndims >= 3 and \
+            ext[0] == 2 and env is not None and \
+            _const_extent(n.func.domain[0], env) == 2 and not no_pairs
         if n.role == 'stage':
             al = max(1, 16 // es)
             whole = env is not None and _const_extent(
@@ -986,7 +1005,7 @@ def _layout_smem(plan, tight=False, env=None, prefetch=False):
                 w = ((ext[-1] + al - 1 + al - 1) // al) * al
             n.pad_inner = w
             ext[-1] = w
-        elif es == 4 and ext[-1] % 4 and ext[-1] > 4:
+        elif es == 4 and ext[-1] % 4 and ext[-1] > 4 and not n.pairs:
             # rows of whole 16-byte chunks, so that the interior path can
             # read four consecutive points with one vector load
             n.pad_inner = ((ext[-1] + 3) // 4) * 4
@@ -1058,6 +1077,64 @@ def _gather_map(pipeline, f, rvars):
     return tmap
 
 
+MAX_CELL_BINS = 64
+
+
+def _cell_map(pipeline, f, fns_all, threads, env):
+    """The grid-cell form of a sum over an image: every part adds into the
+    cell ``[.., c + x / k0, d + y / k1, ..]`` of the point (x, y), in a bin
+    given by the other target dimensions, constant or data-dependent over
+    at most MAX_CELL_BINS bins in all (the bilateral grid: 8 x 8 pixels, 2
+    x 14 bins).  All points of a cell then belong to the k1 threads of one
+    warp that own its columns, so each thread sums into bins of its own
+    without atomics, and the warp adds them up.  None for other sums
+    (option 'no_cells' keeps the atomic form)."""
+    from .pipe import body_parts
+    rv = f.reductionVariables
+    if len(rv) != 2 or 'no_cells' in pipeline.options or \
+            f.typ.size() not in (4, 8) or threads % 32:
+        return None
+    if any(red.op_type != C.Op.Sum for _, _, red in body_parts(f)):
+        return None
+    d = Value.numericToValue(f.default)
+    if not (isinstance(d, Value) and d.value == 0):
+        return None
+    ks, dims, bins = [None, None], [None, None], {}
+    for t, dom in enumerate(f.domain):
+        kinds = set(fns[t].kind for fns in fns_all)
+        if kinds == {'mono'}:
+            keys = set(fns[t].key() for fns in fns_all)
+            fn = fns_all[0][t]
+            e = fn.expr
+            if isinstance(e, AbstractBinaryOpNode) and e.op == '+':
+                l, r = (Value.numericToValue(q) for q in (e.left, e.right))
+                e = r if isinstance(l, Value) else \
+                    l if isinstance(r, Value) else None
+            if len(keys) != 1 or not isinstance(e, AbstractBinaryOpNode) or \
+                    e.op != '/' or e.left is not fn.var or \
+                    ks[fn.cdim] is not None:
+                return None
+            k = Value.numericToValue(e.right)
+            if not (isinstance(k, Value) and isinstance(k.value, int)):
+                return None
+            ks[fn.cdim], dims[fn.cdim] = k.value, t
+        else:
+            ext = _const_extent(dom, env)
+            if ext is None or 'mono' in kinds:
+                return None
+            bins[t] = int(ext)
+    if None in ks or not 2 <= ks[0] <= 32 or ks[1] not in (2, 4, 8, 16, 32):
+        return None
+    for dom, k in zip(f.reductionDomain, ks):
+        lo = try_eval_int(dom.lowerBound, {})
+        if lo is None or lo % k or lo < 0:
+            return None
+    total = int(np.prod(list(bins.values()) or [1]))
+    if total > MAX_CELL_BINS:
+        return None
+    return tuple(ks), tuple(dims), bins
+
+
 def plan_reduction(pipeline, comps):
     from .pipe import body_parts
     if len(comps) != 1:
@@ -1096,6 +1173,13 @@ def plan_reduction(pipeline, comps):
                 ext = try_eval_int(dom.upperBound - dom.lowerBound + 1, env)
                 if ext is not None:
                     plan.tile[d] = max(plan.tile[d], min(int(ext), 1 << 20))
+        return plan
+    plan.cells = _cell_map(pipeline, f, fns_all, plan.threads, env)
+    if plan.cells is not None:
+        (k0, _), _, bins = plan.cells
+        plan.tile = [max(1, plan.tile[0] // k0) * k0, plan.threads]
+        plan.smem_bytes = f.typ.size() * plan.threads * int(
+            np.prod(list(bins.values()) or [1]))
         return plan
     # privatized footprint of one tile, by simulation over a period
     divs = []
