@@ -21,12 +21,9 @@ group (option fuse_all; the greedy grouping leaves six kernels: 0.133 vs
 0.190 ms) and tiles its three output channels whole (option channel_tile:
 a thread computes a pixel's red, green and blue once for all three
 channels, 0.085 vs 0.130 ms) on 32x128 tiles with 4 rows per thread.
-Harris and both pyramids ask ptxas for 4 resident CTAs per SM
-(``min_blocks=4``: at most 64 registers a thread), also outside the tuned
-space: 0.0290 vs 0.0303 ms, 0.203 vs 0.209 ms and
-0.218 vs 0.227 ms (the 8-level pyramid with its interior tiles reading
-clamped taps unclamped); unsharp is bound by shared memory, not
-registers.
+The L=4 pyramid asks ptxas for 4 resident CTAs per SM (``min_blocks=4``:
+at most 64 registers a thread), also outside the tuned space (0.203 vs
+0.209 ms); unsharp is bound by shared memory, not registers.
 The widening pipelines' settings are the best of smaller sweeps
 (polymage_b200.apps.measure, same timing): Jacobi 2-D 32x64 tiles with 5
 steps per group (0.133 vs 0.207 ms for 16x64 with 10), Jacobi 3-D and the
@@ -47,8 +44,8 @@ A later sweep of the CTA-shape knobs (same timing, one box): the camera
 pipe with 3 resident CTAs asked of ptxas (0.0491 vs 0.0553 ms), the L=4
 pyramid with 4 rows per thread and its tile regions computed by one
 thread (option shared_regions: 0.1735 vs 0.1875 ms; every other pipeline
-is slower with that option), the L=8 pyramid and the local Laplacian with
-4 rows per thread (0.2164 vs 0.2237 ms, 0.1474 vs 0.1496 ms),
+is slower with that option), the local Laplacian with 4 rows per thread
+(0.1474 vs 0.1496 ms),
 interpolation with its four channels tiled whole (option channel_tile_all:
 the channels share the alpha channel's work) on 16x64 tiles (0.172 vs
 0.299 ms; 0.181 on 32x64, 0.208 on 8x64).  Harris sums
@@ -86,8 +83,11 @@ BILATERAL = dict(tile_sizes=(1, 32, 128), group_size=10,
 PYRAMID = dict(tile_sizes=(32, 64), group_size=10,
                options=('rblock=4', 'min_blocks=4', 'shared_regions'))
 # 8 levels, indices clamped at every level's borders (any image size)
-PYRAMID8 = dict(L=8, tile_sizes=(32, 64), group_size=10,
-                options=('rblock=4', 'min_blocks=4'))
+# (16x64 tiles in CTAs of 128 threads: its coarse levels are a few CTAs
+# whose own latency counts; on the device 0.193 vs 0.206 ms on 32x64 with
+# 256 threads at 2048^2, 0.082 vs 0.087 at 256^2)
+PYRAMID8 = dict(L=8, tile_sizes=(16, 64), group_size=10,
+                options=('rblock=4', 'threads=128'))
 
 # local Laplacian filter (the video demo's pipeline_laplacian), 1080p frames
 # (option tight_stage: the uint8 [x][y][3] frame is staged without the TMA

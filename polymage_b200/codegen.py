@@ -74,6 +74,8 @@ _INT_T = (C.Int, C.UInt, C.Short, C.UShort, C.Char, C.UChar, C.Long,
 # concurrent streams of the single-image entry points (option 'streams=N';
 # 1 launches every group on the caller's stream)
 DEFAULT_STREAMS = 4
+# points that a thread computes at once on interior tiles
+MAX_BLOCK = 20
 
 
 class CodegenError(Exception):
@@ -3433,8 +3435,21 @@ class StencilGen(object):
         none is a strided HBM read (decided by generating the loop once
         into a scratch buffer)."""
         pg = self.pg
-        if 'no_vec' in pg.p.options or ext[-1] % 4 or ext[-1] < 16 or \
+        # rows of a shared-memory stage are padded to 16 bytes: a last
+        # partial vector also computes the padding, from whatever lies
+        # beside the producers' rows, and nothing reads it
+        if 'no_vec' in pg.p.options or ext[-1] < 16 or \
+                ext[-1] % 4 and not (n.role == 'smem' and n.pad_inner) or \
                 n.pairs or n.ndims - 1 in self.cover(n):
+            return 1
+        # That pays where a vector read serves several taps along the row
+        # (Sobel: 18.1 vs 21.5 us for Harris 2048^2 in all).  A filter
+        # across rows reads as many words either way, in fewer and longer
+        # turns of fewer threads (the pyramids' decimation: 216 vs 206 us)
+        if ext[-1] % 4 and not any(
+                len(set(fn.key() for fn in per_dim[-1])) > 1
+                for n2, per_dim in self.inline_uses(n)
+                if n2.in_smem and per_dim):
             return 1
         self.inner_residues()
         if f not in self._loop_res:
@@ -3454,6 +3469,8 @@ class StencilGen(object):
             self.vec_stats = None
         if ok:
             return 4
+        if ext[-1] % 4:
+            return 1
         # 2 points per thread when the stage decides something by the
         # parity of its innermost index (an upsampling by 2 reading x / 2
         # and selecting on x % 2): each of the two points then has a known
@@ -3634,6 +3651,18 @@ class StencilGen(object):
         self.gen_point(f, n)
         w.close()
 
+    def row_parity(self, n):
+        """Whether step node ``n`` or a stage that it evaluates in
+        registers divides its second-innermost index."""
+        from .evaluate import divisors_in
+        d = n.ndims - 2
+        if _inner_parity(n.func, n.func.variables[d]):
+            return True
+        return any(fn.kind == 'mono' and fn.cdim == d and
+                   divisors_in(fn.expr)
+                   for _, per_dim in self.inline_uses(n)
+                   for fns in per_dim for fn in fns)
+
     def block_shape(self, n, ext):
         """(K, cb): rows along the second-innermost dimension and channels
         along a small outermost one that a thread computes at once (with
@@ -3641,31 +3670,37 @@ class StencilGen(object):
         pg = self.pg
         nd = n.ndims
         rb_max = int(_opt(pg.p, 'rblock', 4))
-        K = 1
-        if nd >= 2:
-            outer = ext[-2]
-            # block height: fewest rows loaded (block + a 2-row halo) per
-            # row computed; a last partial block is shifted back to end at
-            # the last row (its overlap is recomputed, same values)
-            best = None
-            for k in range(min(rb_max, outer), 0, -1):
-                cost = -(-outer // k) * (k + 2)
-                if best is None or cost < best:
-                    K, best = k, cost
         # a small outermost dimension (channels) is computed by the same
         # thread, so that reads and index arithmetic shared by the channels
         # of a point are done once
         cb = 1
         if nd >= 3 and ext[0] <= 4 and 'no_cblock' not in pg.p.options:
             cb = ext[0]
-            while K > 1 and K * cb > 16:
-                K -= 1
         V = self.vec if nd >= 2 else 1
-        if V > 1:
-            # 4 consecutive inner points per thread: shared-memory reads of
-            # a row become 16-byte vector loads
-            while K > 1 and K * cb * V > 16:
-                K -= 1
+        K = 1
+        if nd >= 2:
+            # block height: the fewest rows loaded (block + a 2-row halo)
+            # by a thread over all its blocks, at most 20 points a block; a
+            # last partial block is shifted back to end at the last row
+            # (its overlap is recomputed, same values)
+            outer = ext[-2]
+            cols = -(-ext[-1] // V)
+            for d, e in enumerate(ext[:-2]):
+                cols *= 1 if (d == 0 and cb > 1) else e
+            ks = [k for k in range(min(rb_max, outer), 0, -1)
+                  if k == 1 or k * cb * V <= MAX_BLOCK]
+            # rows that are decimated or interpolated (an index divides by
+            # 2): an even height from an even row gives each row of the
+            # block a known parity
+            if any(k % 2 == 0 and outer % k == 0 for k in ks) and \
+                    self.row_parity(n):
+                ks = [k for k in ks if k % 2 == 0 and outer % k == 0]
+            best = None
+            for k in ks:
+                turns = -(-(-(-outer // k) * cols) // self.plan.threads)
+                cost = turns * (k + 2)
+                if best is None or cost < best:
+                    K, best = k, cost
         return K, cb
 
     def gen_fast_box(self, f, n, ext, blk):
@@ -3696,7 +3731,11 @@ class StencilGen(object):
                 d, org, d, org, B - 1, B, B))
             w("int f_hi%d = %s + pm_floordiv(v_hi%d + 1 - %s, %d) * %d - 1;"
               % (d, org, d, org, B, B))
-            if ext[d] % B:
+            if ext[d] % B and d == nd - 1:
+                # a last vector that reaches into the row's padding
+                w("if (v_hi%d >= %s + %d) f_hi%d = %s + %d;" % (
+                    d, org, ext[d] - 1, d, org, -(-ext[d] // B) * B - 1))
+            elif ext[d] % B:
                 w("if (v_hi%d >= %s + %d) f_hi%d = %s + %d;" % (
                     d, org, ext[d] - 1, d, org, ext[d] - 1))
                 w("if (f_lo%d > %s + %d) f_hi%d = f_lo%d - 1;" % (
@@ -3775,7 +3814,8 @@ class StencilGen(object):
             self.vec_res = self._loop_res[f]
         nblk = -(-outer // K)
         rest = ext[:-2] if nd >= 2 else []
-        total = nblk * (inner // V)
+        nvec = -(-inner // V)
+        total = nblk * nvec
         for d, e in enumerate(rest):
             total *= 1 if (d == 0 and cb > 1) else e
         strides = []
@@ -3787,7 +3827,7 @@ class StencilGen(object):
             "if (%s) " % box if box else "", total, plan.threads))
         if V > 1:
             w("const int ji = (it %% %d) * %d; int rr = it / %d;" % (
-                inner // V, V, inner // V))
+                nvec, V, nvec))
         else:
             w("const int ji = it %% %d; int rr = it / %d;" % (inner, inner))
         if nd >= 2:
@@ -3933,8 +3973,19 @@ class StencilGen(object):
                                   vt, nm, "ib + %d" % (off - 1), vt, k, u,
                                   v))
                         continue
-                    self._store(f, n, qs, v, flag, idx, gidx,
+                    svec = None
+                    if V == 4 and n.in_smem and f.typ.size() == 4 and \
+                            all(st % 4 == 0 for st in strides[:-1]):
+                        svec = {'float': 'float4',
+                                'int': 'int4'}.get(ctype(f.typ))
+                    self._store(f, n, qs, v, flag,
+                                None if svec else idx, gidx,
                                 hbm=vst is None)
+                    if svec and u == V - 1:
+                        w("*reinterpret_cast<%s*>(&sm_%s[%s]) = make_%s(%s);"
+                          % (svec, nm, "ib + %d" % (off - u), svec,
+                             ", ".join("v%d_%d_%d" % (c, k, i)
+                                       for i in range(V))))
                     if vst is None:
                         continue
                     group.append((qs, v, flag, gidx))
