@@ -26,14 +26,15 @@ at most 64 registers a thread), also outside the tuned space (0.203 vs
 0.209 ms); unsharp is bound by shared memory, not registers.
 The widening pipelines' settings are the best of smaller sweeps
 (polymage_b200.apps.measure, same timing): Jacobi 2-D 32x64 tiles with 5
-steps per group (0.133 vs 0.207 ms for 16x64 with 10), Jacobi 3-D and the
+steps per group (0.133 vs 0.207 ms for 16x64 with 10) and up to 8 rows per
+thread (0.101 vs 0.106 ms with 4), Jacobi 3-D and the
 3-D multigrid cycles unfused (group size 1; 0.164 vs 0.356 ms and 3.2 vs
 8.6 ms on the larger tiles of that sweep): in 3-D the halo of a fused time
 step grows every face of a tile, so recomputation costs more than the HBM
-round trip it saves.  Their tiles are small, 4x16x32 and 4x8x32 points in
-CTAs of 128 threads, four to nine of which reside on an SM, so that some
-load while others compute (Jacobi 3-D 128^3 0.117 vs 0.139 ms on 8x16x32
-with 256 threads, V-cycle 255^3 1.37 vs 1.96 ms on 8x16x64 with 256;
+round trip it saves.  Their tiles are small, 4x8x32 points in CTAs of 128
+threads, nine of which reside on an SM, so that some load while others
+compute (Jacobi 3-D 128^3 0.107 vs 0.117 ms on 4x16x32 and 0.139 on 8x16x32
+with 256 threads; 2x8x32 is faster below 64^3 only; V-cycle 255^3 1.37 vs 1.96 ms on 8x16x64 with 256;
 4x8x64 and 8x8x64 lie between, tiles 34 or 66 wide, which cover 2^k + 2
 points without a remainder, behind).  The Jacobi steps, the multigrid cycles
 and NAS MG also stage their pointwise-read right-hand sides by TMA (option
@@ -104,8 +105,8 @@ LAPLACIAN = dict(tile_sizes=(32, 64), group_size=10,
 INTERPOLATE = dict(rows=2048, cols=2048, tile_sizes=(16, 64), group_size=11,
                    options=('channel_tile_all',))
 JACOBI2D = dict(N=2048, T=10, tile_sizes=(32, 64), group_size=5,
-                options=('stage_pointwise',))
-JACOBI3D = dict(N=128, T=10, tile_sizes=(4, 16, 32), group_size=1,
+                options=('stage_pointwise', 'rblock=8'))
+JACOBI3D = dict(N=128, T=10, tile_sizes=(4, 8, 32), group_size=1,
                 options=('stage_pointwise', 'threads=128'))
 VCYCLE = dict(n=31, L=3, nu1=10, nu2=0, nuc=0, tile_sizes=(8, 32),
               group_size=6, options=('stage_pointwise',))
