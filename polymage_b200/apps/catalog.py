@@ -86,9 +86,11 @@ PYRAMID = dict(tile_sizes=(32, 64), group_size=10,
 # 8 levels, indices clamped at every level's borders (any image size)
 # (16x64 tiles in CTAs of 128 threads: its coarse levels are a few CTAs
 # whose own latency counts; on the device 0.193 vs 0.206 ms on 32x64 with
-# 256 threads at 2048^2, 0.082 vs 0.087 at 256^2)
+# 256 threads at 2048^2, 0.082 vs 0.087 at 256^2; the two images' and the
+# mask's level in one launch, option merge_launches: a call takes 0.201 vs
+# 0.207 ms at 2048^2, 0.085 vs 0.119 at 256^2)
 PYRAMID8 = dict(L=8, tile_sizes=(16, 64), group_size=10,
-                options=('rblock=4', 'threads=128'))
+                options=('rblock=4', 'threads=128', 'merge_launches'))
 
 # local Laplacian filter (the video demo's pipeline_laplacian), 1080p frames
 # (option tight_stage: the uint8 [x][y][3] frame is staged without the TMA

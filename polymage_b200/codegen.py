@@ -3233,8 +3233,12 @@ class StencilGen(object):
         lanes per row so that the row's index arithmetic and its bounds
         tests are done once per row and the copies of a warp are
         contiguous.  Unsharp 3x1079x1917 (rows of 7684 bytes, 68 x 136
-        floats a tile): 21.0 us, against 27.7 us with one element a
-        thread and iteration.  Narrower elements (cp.async moves 4 bytes
+        floats a tile): 21.4 us a cold launch, against 27.7 us with one
+        element a thread and iteration; 17.7 us a call in a row, where
+        1916 columns, which TMA loads, take 12.8: the copies' own issue
+        slots.  A second loop without tests for buffers that lie in the
+        array whole gained unsharp 5 % and cost interpolation 8 %.
+        Narrower elements (cp.async moves 4 bytes
         at least) keep that form."""
         pg = self.pg
         plan = self.plan
@@ -5299,8 +5303,106 @@ def gen_chains(pg, pipeline):
             'kernel': ck, 'members': [sg.k for sg in sgs],
             'phases': phases, 'smem': smem, 'threads': nt})
     # the chains take their members' places in the launch list
+    _replace_launches(pg, replace)
+
+
+def plan_merges(pg, pipeline):
+    """Runs of consecutive stencil launches that one launch replaces
+    (option 'merge_launches'): no two have a read/write hazard, and their
+    CTAs have the same size."""
+    if 'merge_launches' not in pipeline.options or pg.meta.get('chains'):
+        return []
+    runs, cur = [], []
+    for j in range(len(pg.launch_fns)):
+        sg = pg.stencil_of.get(j)
+        ok = sg is not None and not sg.prefetch and j not in pg.launch_main
+        rj, wj = pg.launch_rw[j]
+        fits = ok and cur and all(
+            sg.launch_bounds == pg.stencil_of[i].launch_bounds and
+            not (pg.launch_rw[i][1] & rj or pg.launch_rw[i][0] & wj or
+                 pg.launch_rw[i][1] & wj) for i in cur) and \
+            sum(_launch_param_bytes(pg.stencil_of[i])
+                for i in cur + [j]) <= CHAIN_PARAM_BYTES
+        if not fits:
+            runs.append(cur)
+            cur = []
+        if ok:
+            cur.append(j)
+    runs.append(cur)
+    return [r for r in runs if len(r) > 1]
+
+
+def gen_merges(pg, pipeline):
+    """One kernel per run of independent launches
+    (``pm_<name>_merge<m>``): its CTAs are the members' tiles one member
+    after another.  The 8-level pyramid decimates two images and a mask
+    level by level, three short launches a level on three streams; merged
+    it takes 16 launches on one stream instead of 30, which the host
+    issues about 4.4 us apart (B200, us a call, 256^2 119 -> 85, 1001x1403
+    135 -> 131, 2048^2 207 -> 201)."""
+    runs = plan_merges(pg, pipeline)
+    if not runs:
+        return
+    w = pg.w
+    w("// ---- independent groups in one launch")
+    replace = {}
+    for c, run in enumerate(runs):
+        sgs = [pg.stencil_of[j] for j in run]
+        mk = "pm_%s_merge%d" % (pg.pname, c)
+        nt = sgs[0].plan.threads
+        smem = max(sg.plan.smem_bytes for sg in sgs)
+        w("// %s: %s" % (mk, ", ".join(sg.k for sg in sgs)))
+        w.open("struct %s_launch" % mk)
+        for m, sg in enumerate(sgs):
+            w("%s_launch m%d;" % (sg.k, m))
+        w("int n[%d];           // tiles of each member" % len(sgs))
+        w.close("};")
+        w('extern "C" __global__ void __launch_bounds__(%s) %s(const '
+          '__grid_constant__ %s_launch C)' % (sgs[0].launch_bounds, mk, mk))
+        w.open("")
+        w("int b = (int)blockIdx.x;")
+        for m, sg in enumerate(sgs):
+            w("if (b < C.n[%d]) { %s_body<false>(C.m%d, b, C.n[%d]); return; "
+              "}" % (m, sg.k, m, m))
+            w("b -= C.n[%d];" % m)
+        w.close()
+        w("static bool %s_attr[64];     // per device" % mk)
+        w.open("static int launch_%s(pm_args& A, const size_t* wsoff, "
+               "cudaStream_t s)" % mk)
+        w("%s_launch C; memset(&C, 0, sizeof(C));" % mk)
+        w("long long nt = 0, total = 0;")
+        w("int st = PM_OK;")
+        for m, sg in enumerate(sgs):
+            w("if ((st = fill_%s(C.m%d.d0, A, wsoff, &nt))) return st;" % (
+                sg.k, m))
+            w("if ((total += nt) > 0x7fffffffLL) return PM_ERR_UNSUPPORTED;")
+            w("C.m%d.nimg = 1; C.m%d.total = C.n[%d] = (int)nt;" % (m, m, m))
+        w("if (total == 0) return PM_OK;")
+        w.open("if (!%s_attr[pm_cur_dev()])" % mk)
+        w("if (cudaFuncSetAttribute(%s, cudaFuncAttributeMaxDynamicShared"
+          "MemorySize, %d) != cudaSuccess) return PM_ERR_CUDA;" % (mk, smem))
+        w("%s_attr[pm_cur_dev()] = true;" % mk)
+        w.close()
+        if 'no_pdl' not in pg.p.options:
+            w("if (pm_launch_pdl(%s, (unsigned)total, %d, %d, s, C, %s) != "
+              "cudaSuccess) return PM_ERR_CUDA;" % (
+                  mk, nt, smem, "true" if 'pdl' in pg.p.options else
+                  "false"))
+        else:
+            w("%s<<<(unsigned)total, %d, %d, s>>>(C);" % (mk, nt, smem))
+        w("return cudaGetLastError() == cudaSuccess ? PM_OK : PM_ERR_CUDA;")
+        w.close()
+        w("")
+        replace[run[0]] = ("launch_" + mk, run)
+    pg.meta['merges'] = [[pg.stencil_of[j].k for j in run] for run in runs]
+    _replace_launches(pg, replace)
+
+
+def _replace_launches(pg, replace):
+    """Put launch functions in the places of the runs of launches they
+    stand for ({first launch: (function, launches)})."""
     fns, rw, main = [], [], []
-    member = set(j for run, _ in chains for j in run)
+    member = set(j for _, run in replace.values() for j in run)
     for j in range(len(pg.launch_fns)):
         if j in replace:
             fn, run = replace[j]
@@ -5360,12 +5462,14 @@ def generate_code_for_pipeline(pipeline):
     pg.group_launch_rw = list(pg.launch_rw)
     pg.group_launch_main = list(pg.launch_main)
     gen_chains(pg, pipeline)
+    gen_merges(pg, pipeline)
     # kernel launches of one single-image call (a Reduction: its init
-    # and accumulation; a chain: one for all its members)
+    # and accumulation; a chain or a merge: one for all its members)
     pg.meta['launches'] = sum(
         {'stencil': 1, 'reduction': 2}.get(g.plan.kind, 0)
         for g in pipeline.groups) - sum(
-            len(ch['members']) - 1 for ch in pg.meta.get('chains', []))
+            len(ch['members']) - 1 for ch in pg.meta.get('chains', [])) - sum(
+                len(run) - 1 for run in pg.meta.get('merges', []))
     pg.w = pg_w
     w = pg.w
     w("// pipeline %s -- generated by polymage_b200 for sm_100a" %

@@ -37,7 +37,8 @@ as ``"name=value"`` strings or ``(name, value)`` tuples:
   for the caller's stream only), ``pdl`` / ``no_pdl`` (programmatic stream
   serialization also in captured graphs / nowhere), ``chain`` / ``('chain', N)`` (consecutive stencil groups
   of at most N tiles each as phases of one launch, grid barriers between
-  dependent phases);
+  dependent phases), ``merge_launches`` (consecutive independent stencil
+  groups as one launch);
 * switches of single optimisations, for measurement and debugging:
   ``shared_regions`` (one thread computes a tile's regions and shares
   them through shared memory), ``no_inside`` (every tile on the general
