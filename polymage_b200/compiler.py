@@ -41,8 +41,9 @@ as ``"name=value"`` strings or ``(name, value)`` tuples:
   groups as one launch);
 * switches of single optimisations, for measurement and debugging:
   ``shared_regions`` (one thread computes a tile's regions and shares
-  them through shared memory), ``no_inside`` (every tile on the general
-  path), ``guarded`` (one point per iteration), ``no_vec``, ``no_vec2``,
+  them through shared memory), ``no_inside`` (every tile
+  point by point, conditions evaluated), ``guarded`` (the same for every
+  stage), ``no_vec``, ``no_vec2``,
   ``no_cblock``, ``no_pairs`` (two channels of a shared-memory stage not
   interleaved), ``no_static_res``, ``no_fold_clamps``.
 """
