@@ -20,7 +20,9 @@ resident CTAs (0.0480 vs 0.0508 ms).  The camera pipe fuses every stage into one
 group (option fuse_all; the greedy grouping leaves six kernels: 0.133 vs
 0.190 ms) and tiles its three output channels whole (option channel_tile:
 a thread computes a pixel's red, green and blue once for all three
-channels, 0.085 vs 0.130 ms) on 32x128 tiles with 4 rows per thread.
+channels, 0.085 vs 0.130 ms) with 4 rows per thread, on 32x64 tiles in
+CTAs of 128 threads, 6 of them asked of ptxas (a call 0.0329 ms, 0.0347 on
+32x128 with 256 threads and 3, 0.0334 on 16x128 with 128 and 6).
 The L=4 pyramid asks ptxas for 4 resident CTAs per SM (``min_blocks=4``:
 at most 64 registers a thread), also outside the tuned space (0.203 vs
 0.209 ms); unsharp is bound by shared memory, not registers.
@@ -41,15 +43,16 @@ and NAS MG also stage their pointwise-read right-hand sides by TMA (option
 stage_pointwise: Jacobi 2-D 0.116 vs 0.132 ms, 3-D 0.117 vs 0.138 ms,
 V-cycle 0.073 vs 0.083 ms, W-cycle 0.138 vs 0.155 ms, NAS MG 0.255 vs
 0.264 ms, 3-D V-cycle 1.17 vs 1.61 ms).
-A later sweep of the CTA-shape knobs (same timing, one box): the camera
-pipe with 3 resident CTAs asked of ptxas (0.0491 vs 0.0553 ms), the L=4
+A later sweep of the CTA-shape knobs (same timing, one box): the L=4
 pyramid with 4 rows per thread and its tile regions computed by one
 thread (option shared_regions: 0.1735 vs 0.1875 ms; every other pipeline
 is slower with that option), the local Laplacian with 4 rows per thread
 (0.1474 vs 0.1496 ms),
 interpolation with its four channels tiled whole (option channel_tile_all:
 the channels share the alpha channel's work) on 16x64 tiles (0.172 vs
-0.299 ms; 0.181 on 32x64, 0.208 on 8x64).  Harris sums
+0.299 ms; 0.181 on 32x64, 0.208 on 8x64) with 2 rows per thread and channel
+(0.141 vs 0.150 ms with 4 on the device: its coarse levels are a few CTAs
+with more threads than blocks).  Harris sums
 its 3x3 box sums and Sobel taps as row sums that the rows of a thread's
 block share (option separable: 0.0255 vs 0.0274 ms).  The 2-D multigrid
 cycles take 8x32 tiles: their 255^2 grids give 16x64 tiles too few CTAs
@@ -75,9 +78,9 @@ HARRIS = dict(tile_sizes=(32, 64), group_size=11,
                        'separable'))
 UNSHARP = dict(tile_sizes=(64, 128), group_size=10,
                options=('rblock=16', 'inline_budget=400', 'threads=128'))
-CAMPIPE = dict(tile_sizes=(32, 128), group_size=12,
+CAMPIPE = dict(tile_sizes=(32, 64), group_size=12,
                options=('rblock=4', 'fuse_all', 'channel_tile',
-                        'min_blocks=3'))
+                        'threads=128', 'min_blocks=6'))
 BILATERAL = dict(tile_sizes=(1, 32, 128), group_size=10,
                  options=(('red_tile', (16, 256)), 'rblock=4',
                           'stage_pointwise', 'min_blocks=3'))
@@ -105,7 +108,7 @@ LAPLACIAN = dict(tile_sizes=(32, 64), group_size=10,
 # (multigrid/jacobi{2D,3D}/Makefile:10-16), NAS MG class W (NAS-PB-MG-3.2/
 # Makefile:9), interpolation of a 2048x2048 RGBA image.
 INTERPOLATE = dict(rows=2048, cols=2048, tile_sizes=(16, 64), group_size=11,
-                   options=('channel_tile_all',))
+                   options=('channel_tile_all', 'rblock=2'))
 JACOBI2D = dict(N=2048, T=10, tile_sizes=(32, 64), group_size=5,
                 options=('stage_pointwise', 'rblock=8'))
 JACOBI3D = dict(N=128, T=10, tile_sizes=(4, 8, 32), group_size=1,
