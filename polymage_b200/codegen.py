@@ -3487,9 +3487,12 @@ class StencilGen(object):
 
     def vec_read(self, node, f, args):
         """Text of a 16-byte-vector read covering point ``args`` of smem
-        node ``node`` (one lane of a cached float4/int4), or None."""
+        node ``node`` (one lane of a cached float4/int4), or None: also
+        where the channels are interleaved, since the four points of a row
+        then lie 8 bytes apart."""
         ctx = self.ctx
-        if node.func.typ.size() != 4 or not node.in_smem or self.vec != 4:
+        if node.func.typ.size() != 4 or not node.in_smem or \
+                node.pairs or self.vec != 4:
             return None
         res = self.inner_residues()
         if node.func not in res or node._sm_ext[-1] % 4:

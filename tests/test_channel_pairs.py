@@ -1,0 +1,60 @@
+"""Two-channel stages whose channels are interleaved in shared memory,
+read by the forms that know the layout and by those that do not: the
+kernels of small pipelines run on the CPU (tests/emulate.py, which refuses
+misaligned and out-of-bounds accesses) against the point-by-point
+evaluation of their definitions."""
+
+import numpy as np
+import pytest
+
+from polymage_b200.compiler import buildPipeline
+from polymage_b200.constructs import (Cast, Float, Function, Image, Int,
+                                      Interval, Parameter, Variable)
+from tests import emulate
+from tests.dsl_eval import Evaluator
+
+R, C = Parameter(Int, "R"), Parameter(Int, "C")
+x, y, c = (Variable(Int, n) for n in "xyc")
+ROWS, COLS = Interval(Int, 1, R), Interval(Int, 1, C)
+CH = Interval(Int, 0, 1)
+
+
+def _filtered(typ):
+    """A two-channel stage that is kept in shared memory."""
+    img = Image(typ, "img", [2, R + 4, C + 4])
+    f = Function(([c, x, y], [CH, Interval(Int, 0, R + 2),
+                              Interval(Int, 0, C + 2)]), typ, "f")
+    f.defn = [img(c, x, y) + 2 * img(c, x + 1, y + 1)]
+    return img, f
+
+
+def _build(out, name, tile, *options):
+    p = buildPipeline([out], param_estimates=[(R, 500), (C, 500)],
+                      tile_sizes=list(tile), pipe_name=name,
+                      options=['inline_budget=0'] + list(options))
+    f, = [n for g in p.groups for n in g.plan.nodes if n.name == "f"]
+    assert f.role == 'smem'
+    return p, f
+
+
+def _check(p, inputs, sizes, tmp_path):
+    prm = {'R': sizes[0], 'C': sizes[1]}
+    got = emulate.run(p, prm, inputs, tmp_path)
+    ev = Evaluator(prm, inputs)
+    for out in p.ordered_params()[2]:
+        ref = ev.array(out)
+        # float32 sums of at most six products of values below 3
+        assert np.abs(got[out.name] - ref).max() <= 32 * 2.0 ** -23
+
+
+def test_data_dependent_channel(tmp_path):
+    img, f = _filtered(Float)
+    m = Image(Int, "m", [R + 4, C + 4])
+    g = Function(([x, y], [ROWS, COLS]), Float, "g")
+    ch = Cast(Int, m(x, y))
+    g.defn = [f(ch, x - 1, y) + f(ch, x + 1, y)]
+    p, _ = _build(g, "pairs_dd", (16, 64), 'stage_pointwise')
+    rng = np.random.default_rng(1)
+    _check(p, {'img': rng.random((2, 41, 94)).astype(np.float32),
+               'm': rng.integers(0, 2, (41, 94)).astype(np.int32)},
+           (37, 90), tmp_path)
