@@ -962,6 +962,19 @@ def _alignment(plan, env):
                     raise PlanError("inconsistent scaling of %s" % n.name)
 
 
+def _both_channels(n):
+    """Whether the outermost dimension is two channels and every tile's
+    region holds both: a pair is addressed from the first channel, so a
+    region that starts at the second (a tile of channel 1 that reads only
+    its own) would put it one element below its 8-byte boundary."""
+    lo = try_eval_int(n.func.domain[0].lowerBound, {})
+    hi = try_eval_int(n.func.domain[0].upperBound, {})
+    if lo is None or hi != lo + 1 or 0 not in n.const_bounds:
+        return False
+    a, b = n.const_bounds[0]
+    return bool(np.all(a == lo) and np.all(b == hi))
+
+
 def _layout_smem(plan, tight=False, env=None, prefetch=False,
                  no_pairs=False):
     """Shared-memory buffers, placed first-fit by lifetime.  A staged
@@ -992,8 +1005,7 @@ def _layout_smem(plan, tight=False, env=None, prefetch=False,
         # lane by lane instead of 16 words (50.8 vs 52.7 us a call at
         # 2560x1536; option 'no_pairs' keeps the planes apart)
         n.pairs = n.role == 'smem' and es == 4 and n.ndims >= 3 and \
-            ext[0] == 2 and env is not None and \
-            _const_extent(n.func.domain[0], env) == 2 and not no_pairs
+            env is not None and _both_channels(n) and not no_pairs
         if n.role == 'stage':
             al = max(1, 16 // es)
             whole = env is not None and _const_extent(

@@ -58,3 +58,17 @@ def test_data_dependent_channel(tmp_path):
     _check(p, {'img': rng.random((2, 41, 94)).astype(np.float32),
                'm': rng.integers(0, 2, (41, 94)).astype(np.int32)},
            (37, 90), tmp_path)
+
+
+def test_tiles_of_one_channel(tmp_path):
+    """Tiles of channel 1 read only that channel of the stage: its region
+    does not start at the domain's first one."""
+    img, f = _filtered(Float)
+    g = Function(([c, x, y], [CH, ROWS, COLS]), Float, "g")
+    g.defn = [f(c, x - 1, y) + f(c, x + 1, y) +
+              f(1, x, y - 1) * f(1, x, y + 1)]
+    p, n = _build(g, "pairs_tile", (1, 16, 32))
+    assert n.ext[0] == 2 and not n.pairs
+    rng = np.random.default_rng(2)
+    _check(p, {'img': rng.random((2, 39, 74)).astype(np.float32) / 2},
+           (35, 70), tmp_path)
