@@ -1004,8 +1004,8 @@ def _layout_smem(plan, tight=False, env=None, prefetch=False,
         # grid's slicing gathers 8 pairs a pixel from bins that differ
         # lane by lane instead of 16 words (50.8 vs 52.7 us a call at
         # 2560x1536; option 'no_pairs' keeps the planes apart)
-        n.pairs = n.role == 'smem' and es == 4 and n.ndims >= 3 and \
-            env is not None and _both_channels(n) and not no_pairs
+        n.pairs = n.role == 'smem' and n.ndims >= 3 and \
+            n.func.typ in (C.Float, C.Int) and env is not None and _both_channels(n) and not no_pairs
         if n.role == 'stage':
             al = max(1, 16 // es)
             whole = env is not None and _const_extent(

@@ -9,7 +9,7 @@ import pytest
 
 from polymage_b200.compiler import buildPipeline
 from polymage_b200.constructs import (Cast, Float, Function, Image, Int,
-                                      Interval, Parameter, Variable)
+                                      Interval, Parameter, UInt, Variable)
 from tests import emulate
 from tests.dsl_eval import Evaluator
 
@@ -72,3 +72,25 @@ def test_tiles_of_one_channel(tmp_path):
     rng = np.random.default_rng(2)
     _check(p, {'img': rng.random((2, 39, 74)).astype(np.float32) / 2},
            (35, 70), tmp_path)
+
+
+@pytest.mark.parametrize("typ", [Float, Int, UInt])
+def test_types(typ, tmp_path):
+    """Interleaved channels of every 4-byte type: both channels of a
+    data-dependent bin."""
+    img = Image(typ, "img", [2, R + 4, C + 4, 6])
+    m = Image(Int, "m", [R + 4, C + 4])
+    z = Variable(Int, "z")
+    f = Function(([c, x, y, z], [CH, Interval(Int, 0, R + 2), Interval(
+        Int, 0, C + 2), Interval(Int, 0, 5)]), typ, "f")
+    f.defn = [img(c, x, y, z) + img(c, x + 1, y + 1, z)]
+    g = Function(([x, y], [ROWS, COLS]), typ, "g")
+    k = Cast(Int, m(x, y))
+    g.defn = [f(0, x, y, k) + 3 * f(1, x, y, k) + f(0, x - 1, y, k)]
+    p, n = _build(g, "pairs_" + typ.c_type_name(), (8, 32))
+    rng = np.random.default_rng(3)
+    img_v = rng.random((2, 21, 54, 6)) * (.25 if typ is Float else 50)
+    _check(p, {'img': img_v.astype(np.float32 if typ is Float else
+                                   np.int64),
+               'm': rng.integers(0, 6, (21, 54)).astype(np.int32)},
+           (17, 50), tmp_path)
