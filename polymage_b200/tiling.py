@@ -962,6 +962,15 @@ def _alignment(plan, env):
                     raise PlanError("inconsistent scaling of %s" % n.name)
 
 
+def _gathered(n):
+    """Whether a consumer reads the node's channels at a data-dependent
+    index, or all its consumers are such stages (nodes are laid out
+    consumers first)."""
+    return any(not is_data_dependent(fns[0].expr) and any(
+        is_data_dependent(fn.expr) for fn in fns[1:]) for _, fns in n.uses) \
+        or bool(n.uses) and all(m.pairs for m, _ in n.uses)
+
+
 def _both_channels(n):
     """Whether the outermost dimension is two channels and every tile's
     region holds both: a pair is addressed from the first channel, so a
@@ -1003,9 +1012,12 @@ def _layout_smem(plan, tight=False, env=None, prefetch=False,
         # 8-byte word (dims [c][..][z] at strides 1, .., 2).  The bilateral
         # grid's slicing gathers 8 pairs a pixel from bins that differ
         # lane by lane instead of 16 words (50.8 vs 52.7 us a call at
-        # 2560x1536; option 'no_pairs' keeps the planes apart)
+        # 2560x1536; option 'no_pairs' keeps the planes apart).  Only for
+        # such gathers and for the stages that feed them alone: a filter
+        # along rows reads the planes by 16-byte vectors instead.
         n.pairs = n.role == 'smem' and n.ndims >= 3 and \
-            n.func.typ in (C.Float, C.Int) and env is not None and _both_channels(n) and not no_pairs
+            n.func.typ in (C.Float, C.Int) and env is not None and _gathered(n) and _both_channels(n) and \
+            not no_pairs
         if n.role == 'stage':
             al = max(1, 16 // es)
             whole = env is not None and _const_extent(
