@@ -3793,8 +3793,13 @@ class StencilGen(object):
         nd = n.ndims
         for d in range(nd):
             if n.role == 'smem' and d in self.cover(n):
-                # zero outside the covered part, which is filled already
-                w("const int s_lo%d = v_lo%d, s_hi%d = v_hi%d;" % ((d,) * 4))
+                # zero outside the covered part, which is filled already;
+                # all of that part, not what of it the unconditional form
+                # can take (a clamp that binds, a stage in registers with
+                # another Case)
+                o, cnt = self.cover(n)[d]
+                w("const int s_lo%d = r_%s_lo%d + %d, s_hi%d = s_lo%d + %d;" %
+                  (d, nm, d, o, d, d, cnt - 1))
                 continue
             top = "pm_imin(r_%s_hi%d, d_%s_hi%d)" % (nm, d, fnm, d)
             if self.needed(n)[d] is not None:
