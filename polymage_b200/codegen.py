@@ -65,7 +65,8 @@ from .expression import substitute_vars, getType, affine_form
 from .bounds import part_boxes
 from .pipe import body_parts
 from .tiling import is_data_dependent
-from .evaluate import EvalError, eval_int, monotone_dir, is_min_max
+from .evaluate import (EvalError, eval_int, monotone_dir, clamp_arm, clamps,
+                       has_clamp, strip_clamps)
 
 _INT_T = (C.Int, C.UInt, C.Short, C.UShort, C.Char, C.UChar, C.Long,
           C.ULong)
@@ -578,28 +579,8 @@ def _has_loop_var(e):
 
 
 def _clamp_arm(e):
-    """The unclamped arm of a clamp ``min/max(v, bound)`` in index
-    arithmetic (``bound`` free of loop variables, no data), else None."""
-    if not is_min_max(e) or is_data_dependent(e):
-        return None
-    t, f = e.true_expression, e.false_expression
-    tv, fv = _has_loop_var(t), _has_loop_var(f)
-    if tv and not fv:
-        return t
-    if fv and not tv:
-        return f
-    return None
-
-
-def _has_clamp(e):
-    stack = [e]
-    while stack:
-        n = stack.pop()
-        if _clamp_arm(n) is not None:
-            return True
-        if hasattr(n, 'children'):
-            stack.extend(n.children())
-    return False
+    """The unclamped arm of a clamp in an index free of data, else None."""
+    return None if is_data_dependent(e) else clamp_arm(e)
 
 
 def _uniform_quotient(e):
@@ -619,36 +600,6 @@ def _uniform_quotient(e):
                 getType(x) in (C.Float, C.Double))
         return False, False
     return ok(e) == (True, True)
-
-
-def _clamps(e):
-    """(arm, bound, is_min) of every clamp ``min/max(arm, bound)`` in an
-    index."""
-    out = []
-    stack = [e]
-    while stack:
-        n = stack.pop()
-        arm = _clamp_arm(n)
-        if arm is not None:
-            t, f, c = n.true_expression, n.false_expression, n.condition
-            less = c.conditional in ('<', '<=')
-            straight = (str(c.lhs), str(c.rhs)) == (str(t), str(f))
-            out.append((arm, f if arm is t else t, less == straight))
-        if hasattr(n, 'children'):
-            stack.extend(n.children())
-    return out
-
-
-def _strip_clamps(e):
-    """Index ``e`` with its clamps replaced by their arms."""
-    arm = _clamp_arm(e)
-    if arm is not None:
-        return _strip_clamps(arm)
-    if isinstance(e, AbstractBinaryOpNode):
-        a, b = _strip_clamps(e.left), _strip_clamps(e.right)
-        return {'+': lambda: a + b, '-': lambda: a - b,
-                '*': lambda: a * b, '/': lambda: a / b}[e.op]()
-    return e
 
 
 class _ArmFn(object):
@@ -2427,8 +2378,8 @@ class StencilGen(object):
                 for d, fns in enumerate(per_dim):
                     ls, hs = [], []
                     for fn in fns:
-                        if fn.kind == 'mono':
-                            t = [ctx.unclamped(fn.expr, {fn.var: b})
+                        if fn.kind == 'mono' and not fn.whole:
+                            t = [self.region_end(n, d, fn, b)
                                  for b in mb[fn.cdim]]
                             if fn.dir < 0:
                                 t.reverse()
@@ -2542,7 +2493,7 @@ class StencilGen(object):
                     mn = self.node_name(m)
                     for fns in per_dim:
                         for fn in fns:
-                            if fn.kind != 'mono' or not _has_clamp(fn.expr):
+                            if fn.kind != 'mono' or not has_clamp(fn.expr):
                                 continue
                             for end in ("lo", "hi"):
                                 b = {fn.var: "r_%s_%s%d" % (mn, end,
@@ -2558,6 +2509,18 @@ class StencilGen(object):
                 conds + ["%s == 0" % t for t in self.shifts] + unclamp) or
                 "false"))
             w("(void)pm_inside;")
+
+    def region_end(self, n, d, fn, end):
+        """C text of index ``fn`` into dimension ``d`` of node ``n`` at an
+        end of its consumer's region: as it is in a dimension of constant
+        extent, without its clamps and rounded down in a parametric one."""
+        ctx = self.ctx
+        if not self.const_dim(n.func, d):
+            return ctx.unclamped(fn.expr, {fn.var: end})
+        ctx.floor_div = False
+        t = ctx.expr(fn.expr, {fn.var: end})
+        ctx.floor_div = True
+        return t
 
     def gen_clamp_shift(self, n):
         """A buffer read through clamped taps holds the clamped positions
@@ -2576,7 +2539,7 @@ class StencilGen(object):
             lo, hi = [], []
             for m, per_dim in self.distinct_uses(n):
                 for fn in per_dim[d]:
-                    if fn.kind == 'mono' and _has_clamp(fn.expr):
+                    if fn.kind == 'mono' and has_clamp(fn.expr):
                         mb = self.use_bounds(m, fn.cdim)
                         t = [ctx.expr(fn.expr, {fn.var: b}) for b in mb]
                         lo.append(t[0 if fn.dir > 0 else 1])
@@ -2604,7 +2567,7 @@ class StencilGen(object):
         envs = [env0] + [dict((k, t) for k in env0) for t in range(1, 65)]
         for m, per_dim in self.distinct_uses(n):
             fns = [fn for fn in per_dim[d]
-                   if fn.kind == 'mono' and _has_clamp(fn.expr)]
+                   if fn.kind == 'mono' and has_clamp(fn.expr)]
             for cdim in set(fn.cdim for fn in fns):
                 dom = m.func.domain[cdim]
                 for env in envs:
@@ -2622,7 +2585,7 @@ class StencilGen(object):
                                 e2[fn.var] = x
                                 diff.append(
                                     eval_int(fn.expr, e2) -
-                                    eval_int(_strip_clamps(fn.expr), e2))
+                                    eval_int(strip_clamps(fn.expr), e2))
                             if min(diff) > 0 or max(diff) < 0:
                                 return False
                     except EvalError:
@@ -2916,9 +2879,9 @@ class StencilGen(object):
                     elif n2.role == 'global' and fn.kind != 'full':
                         require(fn, dom[0], True, dom)
                         require(fn, dom[1], False, dom)
-                    if fn.kind == 'mono' and _has_clamp(fn.expr) and \
+                    if fn.kind == 'mono' and has_clamp(fn.expr) and \
                             'no_fold_clamps' not in pg.p.options:
-                        for arm, bound, is_min in _clamps(fn.expr):
+                        for arm, bound, is_min in clamps(fn.expr):
                             c = _ArmFn(fn, arm)
                             require(c, ctx.expr(bound, {}), not is_min, dom)
         return lo, hi, flags

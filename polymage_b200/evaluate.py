@@ -223,3 +223,61 @@ def monotone_dir(expr, var):
             return a
         return None
     return None
+
+
+def clamp_arm(e):
+    """The unclamped arm of a clamp ``min/max(v, bound)`` in index
+    arithmetic (``bound`` free of loop variables), else None."""
+    if not is_min_max(e):
+        return None
+    t, f = e.true_expression, e.false_expression
+    tv, fv = _has_loop_var(t), _has_loop_var(f)
+    if tv and not fv:
+        return t
+    if fv and not tv:
+        return f
+    return None
+
+
+def has_clamp(e):
+    stack = [e]
+    while stack:
+        n = stack.pop()
+        if clamp_arm(n) is not None:
+            return True
+        if hasattr(n, 'children'):
+            stack.extend(n.children())
+    return False
+
+
+def clamps(e):
+    """(arm, bound, is_min) of every clamp ``min/max(arm, bound)`` in an
+    index."""
+    out = []
+    stack = [e]
+    while stack:
+        n = stack.pop()
+        arm = clamp_arm(n)
+        if arm is not None:
+            t, f, c = n.true_expression, n.false_expression, n.condition
+            less = c.conditional in ('<', '<=')
+            straight = (str(c.lhs), str(c.rhs)) == (str(t), str(f))
+            out.append((arm, f if arm is t else t, less == straight))
+        if hasattr(n, 'children'):
+            stack.extend(n.children())
+    return out
+
+
+def strip_clamps(e):
+    """Index ``e`` with its clamps replaced by their arms."""
+    arm = clamp_arm(e)
+    if arm is not None:
+        return strip_clamps(arm)
+    if isinstance(e, AbstractUnaryOpNode):
+        a = strip_clamps(e.child)
+        return -a if e.op == '-' else a
+    if isinstance(e, AbstractBinaryOpNode) and e.op in '+-*/':
+        a, b = strip_clamps(e.left), strip_clamps(e.right)
+        return {'+': lambda: a + b, '-': lambda: a - b,
+                '*': lambda: a * b, '/': lambda: a / b}[e.op]()
+    return e

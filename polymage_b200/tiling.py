@@ -52,6 +52,7 @@ from . import constructs as C
 from .expr_ast import Value, AbstractBinaryOpNode, InbuiltFunction
 from .expression import substitute_vars
 from .evaluate import (is_min_max, eval_int, EvalError, monotone_dir, divisors_in,
+                       clamps, has_clamp, strip_clamps,
                        try_eval_int)
 
 SMEM_BUDGET = 200 * 1024       # bytes per CTA we allow a plan to use
@@ -77,6 +78,10 @@ class IndexFn(object):
         self.var = None
         self.cdim = None
         self.dir = 0
+        # without its clamps, and whether they make the dimension whole
+        # (see bind_clamps)
+        self.free = self.expr
+        self.clamped = self.whole = False
         e = self.expr
         if is_data_dependent(e):
             return
@@ -93,12 +98,27 @@ class IndexFn(object):
                 self.cdim = [i for i, v in enumerate(consumer_vars)
                              if v is vs[0]][0]
                 self.dir = d
+                self.clamped = has_clamp(e)
+                if self.clamped:
+                    self.free = strip_clamps(e)
 
-    def evaluate(self, value, env):
+    def bind_clamps(self, dom, consumer_dom, env):
+        """A clamped index into a dimension ``dom`` of constant extent.
+        Regions there are the same on every tile of the other dimensions
+        and hold exactly what the clamped index takes.  That needs the
+        consumer's dimension to be of constant extent too and bounds that
+        are literals; otherwise the region is the whole dimension."""
+        if self.clamped and _const_extent(dom, env) is not None:
+            self.whole = _const_extent(consumer_dom, env) is None or any(
+                b.collect(C.Parameter) for _, b, _ in clamps(self.expr))
+
+    def evaluate(self, value, env, free=False):
+        """The index at ``value`` of its variable; ``free``: without its
+        clamps."""
         e = dict(env)
         if self.var is not None:
             e[self.var] = value
-        return eval_int(self.expr, e)
+        return eval_int(self.free if free else self.expr, e)
 
     def key(self):
         return str(self.expr)
@@ -556,6 +576,9 @@ def plan_stencil(pipeline, comps, tile=None):
                 raise PlanError("internal: consumer %s not materialized"
                                 % m.name)
             fns = [IndexFn(a, m.variables) for a in args]
+            for fn, dom in zip(fns, n.func.domain):
+                if fn.kind == 'mono':
+                    fn.bind_clamps(dom, m.domain[fn.cdim], env)
             n.uses.append((node_of[m], fns))
         for fnl in n.uses:
             for fn, dom in zip(fnl[1], n.func.domain):
@@ -737,8 +760,7 @@ def infer_regions(plan, anchor_box, env, clamp=True, tile_first=None):
     ownership of lower-dimensional live-outs)."""
     if not clamp:
         # unclamped regions model interior tiles far from every border:
-        # parameters are taken huge so that indices clamped to a
-        # parameter-dependent bound (min/max) behave as in the interior
+        # indices count without their clamps, and parameters are huge
         env = dict((k, 1 << 40) for k in env)
     regions = {}
     big = 1 << 60
@@ -782,9 +804,9 @@ def infer_regions(plan, anchor_box, env, clamp=True, tile_first=None):
                 nonempty = nonempty & (np.asarray(mlo[d]) <=
                                        np.asarray(mhi[d]))
             for d, fn in enumerate(fns):
-                if fn.kind == 'mono':
-                    a = fn.evaluate(mlo[fn.cdim], env)
-                    b = fn.evaluate(mhi[fn.cdim], env)
+                if fn.kind == 'mono' and not fn.whole:
+                    a = fn.evaluate(mlo[fn.cdim], env, not fixed[d])
+                    b = fn.evaluate(mhi[fn.cdim], env, not fixed[d])
                     a, b = np.minimum(a, b), np.maximum(a, b)
                 elif fn.kind == 'const':
                     a = b = fn.evaluate(0, env)
@@ -943,11 +965,13 @@ def _alignment(plan, env):
             n.scale = [Fraction(1)] * n.ndims
         for m, fns in n.uses:
             for d, fn in enumerate(fns):
-                if fn.kind != 'mono' or m.align[fn.cdim] is None:
+                if fn.kind != 'mono' or m.align[fn.cdim] is None or \
+                        fn.clamped and _const_extent(n.func.domain[d],
+                                                     env) is not None:
                     continue
                 try:
-                    a = fn.evaluate(base, env)
-                    b = fn.evaluate(base + K, env)
+                    a = fn.evaluate(base, env, free=True)
+                    b = fn.evaluate(base + K, env, free=True)
                 except EvalError:
                     continue
                 s = Fraction(b - a, K).limit_denominator(256) * \
