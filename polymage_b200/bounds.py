@@ -18,8 +18,10 @@ kernel read outside a buffer.
 """
 
 import logging
+import math
+from fractions import Fraction
 
-from .expr_ast import Value
+from .expr_ast import (Value, AbstractBinaryOpNode, AbstractUnaryOpNode)
 from . import constructs as C
 from .expression import affine_form
 from .evaluate import eval_int, EvalError, monotone_dir
@@ -340,3 +342,121 @@ def bounds_check_pass(pipeline):
                         raise TypeError("Reference out of domain", f.name,
                                         str(ref), dim, r, (dlo, dhi))
     pipeline._bounds_checks = checks
+
+
+# ---- integer expressions of parameters, compared for every value ----------
+MAX_QUOTIENTS = 6       # nested divisions that a comparison opens
+
+
+def least_params(pipeline):
+    """{parameter name: least value}, from the extents of inputs and
+    outputs: a call in which one is negative is refused."""
+    out = {}
+    _, ins, outs = pipeline.ordered_params()
+    for f in ins + outs:
+        for d in f.domain:
+            form = affine_form(d.upperBound - d.lowerBound + 1)
+            if form is None or len(form[0]) != 1:
+                continue
+            (p, a), = form[0].items()
+            if a > 0:
+                v = -(form[1] // a)
+                out[str(p)] = max(v, out.get(str(p), v))
+    return out
+
+
+class AtEnd(object):
+    """An integer expression at one end of the range of its variable:
+    ``var`` stands for the expression ``end`` and is at least ``low`` (an
+    expression) there."""
+
+    def __init__(self, expr, var, end, low):
+        self.expr, self.var, self.end, self.low = expr, var, end, low
+
+
+def _enclose(e, depth, least, at=None):
+    """``({term: coefficient}, lo, hi)``: the value of integer expression
+    ``e`` lies in [lo, hi] above that linear form, for all parameters not
+    below ``least`` and whichever way a negative quotient is rounded.
+    Divisions are opened ``depth`` deep; a deeper one, and what is no
+    integer arithmetic, is a term of its own."""
+    if isinstance(e, AtEnd):
+        return _enclose(e.expr, depth, least, e)
+    e = Value.numericToValue(e)
+    if at is not None and e is at.var:
+        return _enclose(at.end, depth, least)
+    if isinstance(e, Value) and isinstance(e.value, int):
+        return {}, Fraction(e.value), Fraction(e.value)
+    if isinstance(e, AbstractUnaryOpNode) and e.op == '-':
+        c, lo, hi = _enclose(e.child, depth, least, at)
+        return dict((k, -v) for k, v in c.items()), -hi, -lo
+    if isinstance(e, AbstractBinaryOpNode):
+        k = Value.numericToValue(e.right)
+        if e.op in '+-':
+            a = _enclose(e.left, depth, least, at)
+            b = _enclose(e.right, depth, least, at)
+            c, s = dict(a[0]), 1 if e.op == '+' else -1
+            for t, v in b[0].items():
+                c[t] = c.get(t, 0) + s * v
+            lo, hi = (b[1], b[2]) if s == 1 else (-b[2], -b[1])
+            return dict((t, v) for t, v in c.items() if v), a[1] + lo, \
+                a[2] + hi
+        if e.op == '*':
+            a = _enclose(e.left, depth, least, at)
+            b = _enclose(e.right, depth, least, at)
+            for p, q in ((a, b), (b, a)):
+                if not q[0] and q[1] == q[2]:
+                    f = q[1]
+                    lo, hi = sorted((p[1] * f, p[2] * f))
+                    return dict((t, v * f) for t, v in p[0].items() if f), \
+                        lo, hi
+        if e.op == '/' and depth > 0 and isinstance(k, Value) and \
+                isinstance(k.value, int) and k.value > 0:
+            c, lo, hi = _enclose(e.left, depth - 1, least, at)
+            k = k.value
+            if not c:           # a number: rounded down, or towards zero
+                return {}, Fraction(math.floor(lo / k)), \
+                    Fraction(max(math.floor(hi / k), math.trunc(hi / k)))
+            r = Fraction(k - 1, k)
+            up = 0 if _not_negative(c, lo, least) or at is not None and \
+                not_negative(e.left, at.var, at.low, least) else r
+            return dict((t, v / k) for t, v in c.items()), lo / k - r, \
+                hi / k + up
+    # (a term in the variable has no counterpart at another end)
+    term = at if at is not None and any(
+        v is at.var for v in e.collect(C.Variable)) else str(e)
+    return {term: Fraction(1)}, Fraction(0), Fraction(0)
+
+
+def _not_negative(coeffs, lo, least):
+    return all(v > 0 and t in least for t, v in coeffs.items()) and \
+        lo + sum(v * least[t] for t, v in coeffs.items()) >= 0
+
+
+def not_negative(e, var, low, least):
+    """Whether ``e`` is provably not negative for ``var`` >= ``low``."""
+    if low is None or monotone_dir(e, var) not in (0, 1):
+        return False
+    at = AtEnd(e, var, low, None)
+    return any(_not_negative(c, lo, least) for c, lo, _ in (
+        _enclose(at, i, least) for i in range(MAX_QUOTIENTS + 1)))
+
+
+def excess(a, b, least):
+    """The least constant that provably bounds ``a - b`` from above for all
+    parameter values (see least_params), or None when the two do not
+    compare."""
+    best = None
+    for i in range(MAX_QUOTIENTS + 1):
+        p = _enclose(a, i, least)
+        for j in range(MAX_QUOTIENTS + 1):
+            q = _enclose(b, j, least)
+            if p[0] == q[0] and (best is None or p[2] - q[1] < best):
+                best = p[2] - q[1]
+    return best
+
+
+def at_most(a, b, least):
+    """Whether ``a <= b`` provably holds for all parameter values."""
+    d = excess(a, b, least)
+    return d is not None and d <= 0

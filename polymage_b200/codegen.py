@@ -66,7 +66,7 @@ from .bounds import part_boxes
 from .pipe import body_parts
 from .tiling import is_data_dependent
 from .evaluate import (EvalError, eval_int, monotone_dir, clamp_arm, clamps,
-                       has_clamp, strip_clamps)
+                       has_clamp)
 
 _INT_T = (C.Int, C.UInt, C.Short, C.UShort, C.Char, C.UChar, C.Long,
           C.ULong)
@@ -2338,8 +2338,8 @@ class StencilGen(object):
         origin residues on border tiles as on interior ones (TMA and the
         cooperative loads fill what lies outside with zeros, and no point
         whose Case holds reads it).  Clamped taps count with their
-        unclamped index: a clamp moves an index towards the domain, which
-        the region intersects, so never out of the region.  Along a
+        unclamped index; where a clamp could then move a tap out of the
+        region, the region is moved (gen_clamp_shift).  Along a
         dimension of constant extent regions stay inside the domain."""
         pg = self.pg
         plan = self.plan
@@ -2400,10 +2400,7 @@ class StencilGen(object):
                 for d, (ls, hs) in enumerate(per):
                     los[d] += [t for t in ls if t not in los[d]]
                     his[d] += [t for t in hs if t not in his[d]]
-            moved = n.in_smem and any(
-                not self.const_dim(n.func, d) and not self.meets_domain(n, d)
-                for d in range(nd))
-            cq = "int" if guarded or moved else "const int"
+            cq = "int" if guarded or n.moved else "const int"
 
             def clampd(d, lo, hi):
                 if self.const_dim(n.func, d) and n.role not in (
@@ -2434,7 +2431,12 @@ class StencilGen(object):
                     if self.const_dim(n.func, d):
                         w("r_%s_lo%d = %s; r_%s_hi%d = %s;" % (
                             nm, d, lo, nm, d, hi))
-            self.gen_clamp_shift(n)
+            if any(q.moved for q in plan.nodes) and (n.in_smem or
+                                                     n.role == 'out'):
+                ctx.floor_div = False
+                self.gen_reads(n)
+                ctx.floor_div = True
+                self.gen_clamp_shift(n)
         ctx.floor_div = False
         # Interior tile: every stage's region lies in its domain, its Cases
         # are decided the same way on the whole region, HBM reads stay in
@@ -2522,75 +2524,72 @@ class StencilGen(object):
         ctx.floor_div = True
         return t
 
-    def gen_clamp_shift(self, n):
-        """A buffer read through clamped taps holds the clamped positions
-        too as long as its region meets the domain.  Where that is not
-        certain (a single tap ``f(max(x - 5, 0))`` over a 4-point tile),
-        the region is moved until it does; such a tile runs on the guarded
-        path only (its origins have other residues)."""
-        if not n.in_smem:
-            return
+    def gen_reads(self, n):
+        """``n_<node>_lo/hi``: the points of a node that the tile's points
+        need, clamps evaluated and inside the domain, and ``e_<node>_lo/hi``:
+        those of them whose Case may hold."""
         w = self.pg.w
         ctx = self.ctx
         nm = self.node_name(n)
-        for d in range(n.ndims):
-            if self.const_dim(n.func, d) or self.meets_domain(n, d):
-                continue
-            lo, hi = [], []
-            for m, per_dim in self.distinct_uses(n):
-                for fn in per_dim[d]:
-                    if fn.kind == 'mono' and has_clamp(fn.expr):
-                        mb = self.use_bounds(m, fn.cdim)
-                        t = [ctx.expr(fn.expr, {fn.var: b}) for b in mb]
-                        lo.append(t[0 if fn.dir > 0 else 1])
-                        hi.append(t[1 if fn.dir > 0 else 0])
+        fnm = self.pg.fn(n.func)
+        nd = n.ndims
+        big = "0x3fffffff"
+        for d in range(nd):
+            if n.func is self.plan.anchor:
+                lo = "pm_imax(a_lo%d, d_%s_lo%d)" % (d, fnm, d)
+                hi = "pm_imin(a_hi%d, d_%s_hi%d)" % (d, fnm, d)
+            elif n.role == 'out':
+                lo, hi = "o_%s_lo%d" % (nm, d), "o_%s_hi%d" % (nm, d)
+            else:
+                lo, hi = big, "-" + big
+            w("int n_%s_lo%d = %s, n_%s_hi%d = %s;" % (nm, d, lo, nm, d, hi))
+        for m, per_dim in self.distinct_uses(n):
+            mn = self.node_name(m)
+            w.open("if (%s)" % " && ".join(
+                "e_%s_lo%d <= e_%s_hi%d" % (mn, d, mn, d)
+                for d in range(m.ndims)))
+            for d, fns in enumerate(per_dim):
+                for fn in fns:
+                    if fn.kind == 'mono':
+                        t = [ctx.expr(fn.expr, {fn.var: "e_%s_%s%d" % (
+                            mn, end, fn.cdim)}) for end in ("lo", "hi")]
+                        if fn.dir < 0:
+                            t.reverse()
+                    elif fn.kind == 'const':
+                        t = [ctx.expr(fn.expr, {})] * 2
+                    else:
+                        t = ["d_%s_lo%d" % (fnm, d), "d_%s_hi%d" % (fnm, d)]
+                    w("n_%s_lo%d = pm_imin(n_%s_lo%d, %s); n_%s_hi%d = "
+                      "pm_imax(n_%s_hi%d, %s);" % (nm, d, nm, d, t[0], nm, d,
+                                                   nm, d, t[1]))
+            w.close()
+        cb = getattr(n, 'case_box', None)
+        for d in range(nd):
+            w("n_%s_lo%d = pm_imax(n_%s_lo%d, d_%s_lo%d); n_%s_hi%d = "
+              "pm_imin(n_%s_hi%d, d_%s_hi%d);" % (nm, d, nm, d, fnm, d, nm, d,
+                                                  nm, d, fnm, d))
+            lo, hi = "n_%s_lo%d" % (nm, d), "n_%s_hi%d" % (nm, d)
+            for e in cb[d][0] if cb else []:
+                lo = "pm_imax(%s, %s)" % (lo, ctx.expr(e, {}))
+            for e in cb[d][1] if cb else []:
+                hi = "pm_imin(%s, %s)" % (hi, ctx.expr(e, {}))
+            w("const int e_%s_lo%d = %s, e_%s_hi%d = %s;" % (nm, d, lo, nm, d,
+                                                            hi))
+
+    def gen_clamp_shift(self, n):
+        """Where clamped taps can lie outside a region that follows the
+        unclamped ones (tiling._clamped_reads), the region is moved until
+        it holds what the tile's points read; such a tile runs on the
+        guarded path only (its origins have other residues)."""
+        w = self.pg.w
+        nm = self.node_name(n)
+        for d in sorted(n.moved):
             t = "pm_sh_%s_%d" % (nm, d)
-            w("const int %s = pm_imax(0, %s - r_%s_hi%d) + pm_imin(0, %s - "
-              "r_%s_lo%d);" % (t, _fold("pm_imax", hi, "0"), nm, d,
-                               _fold("pm_imin", lo, "0"), nm, d))
+            w("const int %s = n_%s_lo%d > n_%s_hi%d ? 0 : pm_imax(0, "
+              "n_%s_hi%d - r_%s_hi%d) + pm_imin(0, n_%s_lo%d - r_%s_lo%d);" %
+              (t, nm, d, nm, d, nm, d, nm, d, nm, d, nm, d))
             w("r_%s_lo%d += %s; r_%s_hi%d += %s;" % (nm, d, t, nm, d, t))
             self.shifts.append(t)
-
-    def meets_domain(self, n, d):
-        """Whether the taps of every consumer point include, along
-        dimension ``d``, one that no clamp moves up and one that no clamp
-        moves down (evaluated at both ends of the consumer's domain over a
-        range of parameter values)."""
-        key = (n, d)
-        memo = self.__dict__.setdefault('_meets', {})
-        if key not in memo:
-            memo[key] = self._meets_domain(n, d)
-        return memo[key]
-
-    def _meets_domain(self, n, d):
-        env0 = self.pg.p.int_env()
-        envs = [env0] + [dict((k, t) for k in env0) for t in range(1, 65)]
-        for m, per_dim in self.distinct_uses(n):
-            fns = [fn for fn in per_dim[d]
-                   if fn.kind == 'mono' and has_clamp(fn.expr)]
-            for cdim in set(fn.cdim for fn in fns):
-                dom = m.func.domain[cdim]
-                for env in envs:
-                    try:
-                        ends = [eval_int(dom.lowerBound, env),
-                                eval_int(dom.upperBound, env)]
-                        if ends[0] > ends[1]:
-                            continue
-                        for x in ends:
-                            diff = []
-                            for fn in fns:
-                                if fn.cdim != cdim:
-                                    continue
-                                e2 = dict(env)
-                                e2[fn.var] = x
-                                diff.append(
-                                    eval_int(fn.expr, e2) -
-                                    eval_int(strip_clamps(fn.expr), e2))
-                            if min(diff) > 0 or max(diff) < 0:
-                                return False
-                    except EvalError:
-                        return False
-        return True
 
     def main_part(self, f):
         """The (box, expression) of a piecewise definition that holds on

@@ -49,11 +49,13 @@ import math
 import numpy as np
 
 from . import constructs as C
-from .expr_ast import Value, AbstractBinaryOpNode, InbuiltFunction
+from .expr_ast import (Value, AbstractBinaryOpNode, AbstractUnaryOpNode,
+                       InbuiltFunction)
 from .expression import substitute_vars
 from .evaluate import (is_min_max, eval_int, EvalError, monotone_dir, divisors_in,
-                       clamps, has_clamp, strip_clamps,
-                       try_eval_int)
+                       clamps, clamp_arm, has_clamp, strip_clamps,
+                       try_eval_int, _has_loop_var)
+from .bounds import AtEnd, at_most, excess, least_params
 
 SMEM_BUDGET = 200 * 1024       # bytes per CTA we allow a plan to use
 DEFAULT_THREADS = 256
@@ -191,6 +193,9 @@ class Node(object):
         self.ext = None               # static extents per dim
         self.pad_inner = None         # padded innermost extent (stage)
         self.pairs = False            # two channels interleaved (smem)
+        # dims whose region has to be moved on some tiles to hold what
+        # clamped taps read (see _clamped_reads)
+        self.moved = set()
         self.smem_off = None
         self.smem_bytes = 0
         self.step = None              # compute step (0: staged inputs)
@@ -599,6 +604,7 @@ def plan_stencil(pipeline, comps, tile=None):
     for n in nodes:
         # materialized consumers read only where their Case holds
         n.case_box = case_box(n.func) if n.role in ('out', 'smem') else None
+    least = least_params(pipeline)
     plan.nodes = nodes
     plan.node_of = node_of
 
@@ -615,6 +621,7 @@ def plan_stencil(pipeline, comps, tile=None):
         n.last_step = last
 
     _static_extents(plan, env)
+    _clamped_reads(plan, env, least)
     _alignment(plan, env)
     _layout_smem(plan, tight=('tight_stage' in pipeline.options), env=env,
                  prefetch=('prefetch' in pipeline.options),
@@ -905,6 +912,8 @@ def _static_extents(plan, env):
         for n in plan.nodes:
             lo, hi = regs[n.func]
             e = []
+            n.least_ext = [int(np.min(np.asarray(hi[d]) - np.asarray(lo[d])))
+                           + 1 for d in range(n.ndims)]
             dom = _domain_vals(n.func, env)
             for d in range(n.ndims):
                 ext = np.max(np.asarray(hi[d]) - np.asarray(lo[d]) + 1)
@@ -940,6 +949,198 @@ def _static_extents(plan, env):
             n.ext = a
         if capped:
             n.ext = [x + 2 for x in n.ext]
+
+
+def _bound_forms(e, sign=1):
+    """[(e with one clamp replaced by its bound, that clamp keeps the index
+    from falling below it)] for every clamp of index ``e``, the others
+    dropped; None where a clamp stands in a form not handled."""
+    arm = clamp_arm(e)
+    if arm is not None:
+        inner = _bound_forms(arm, sign)
+        if inner is None:
+            return None
+        (_, bound, is_min), = [c for c in clamps(e) if c[0] is arm][:1]
+        return [(bound, is_min == (sign < 0))] + inner
+    if isinstance(e, AbstractBinaryOpNode) and e.op in '+-*/':
+        out = []
+        for child, other, s in ((e.left, e.right, 1), (
+                e.right, e.left, -1 if e.op == '-' else 1)):
+            child = Value.numericToValue(child)
+            if not has_clamp(child):
+                continue
+            if e.op in '*/':
+                k = Value.numericToValue(other)
+                if not isinstance(k, Value) or child is not e.left and \
+                        e.op == '/':
+                    return None
+                s = 1 if k.value > 0 else -1
+            inner = _bound_forms(child, sign * s)
+            if inner is None:
+                return None
+            other = strip_clamps(other)
+            for b, low in inner:
+                l, r = (b, other) if child is e.left else (other, b)
+                out.append(({'+': lambda: l + r, '-': lambda: l - r,
+                             '*': lambda: l * r, '/': lambda: l / r}[e.op](),
+                            low))
+        return out
+    return None if has_clamp(e) else []
+
+
+class _Taps(object):
+    """The taps of one consumer into one parametric dimension."""
+
+    def __init__(self, m, fns, least):
+        self.m, self.fns, self.least = m, fns, least
+        cb = getattr(m, 'case_box', None)
+        dom = m.func.domain
+        self.los = [[q.lowerBound] + (list(cb[d][0]) if cb else [])
+                    for d, q in enumerate(dom)]
+        self.his = [[q.upperBound] + (list(cb[d][1]) if cb else [])
+                    for d, q in enumerate(dom)]
+
+    def end(self, fn, low):
+        """The index without its clamps at the end of the consumer's points
+        where it is least (``low``) or greatest; one candidate for each
+        bound of those points."""
+        ends = (self.los if low == (fn.dir > 0) else self.his)[fn.cdim]
+        return [AtEnd(fn.free, fn.var, e, q) for e in ends
+                for q in self.los[fn.cdim]]
+
+    def inside(self):
+        """Whether the unclamped taps of every point enclose its clamped
+        ones."""
+        for fn in self.fns:
+            forms = _bound_forms(fn.expr) if fn.clamped else []
+            if forms is None:
+                return False
+            for b, low in forms:
+                if _has_loop_var(b) or not any(
+                        at_most(b, e, self.least) if low else
+                        at_most(e, b, self.least)
+                        for q in self.fns if q.dir == fn.dir and
+                        q.cdim == fn.cdim for e in self.end(q, low)):
+                    return False
+        return True
+
+    def reach(self, dom):
+        """How much wider than the unclamped taps of one point the taps of
+        a tile can lie, besides those of an unclamped tile: the most by
+        which the clamps of one end, or of both in an image of one tile,
+        lead past the unclamped indices; None when not bounded by a
+        constant.  ``dom``: the producer's dimension, which no tap
+        leaves."""
+        below = above = 0
+        to_hi, to_lo = [], []
+        for fn in self.fns:
+            forms = _bound_forms(fn.expr) if fn.clamped else []
+            if forms is None:
+                return None
+            for b, low in forms:
+                if _has_loop_var(b):
+                    return None
+                far = [excess(b, e, self.least) if low else
+                       excess(e, b, self.least)
+                       for e in self.end(fn, low)]
+                far = [q for q in far if q is not None]
+                if not far:
+                    return None
+                far = int(math.ceil(min(far)))
+                if low:
+                    above = max(above, far)
+                    to_lo.append(excess(b, dom.lowerBound, self.least))
+                else:
+                    below = max(below, far)
+                    to_hi.append(excess(dom.upperBound, b, self.least))
+        both = [below + above] + [int(math.ceil(max(q))) for q in (
+            to_lo, to_hi) if q and None not in q]
+        return max(below, above, min(both))
+
+
+def _spread(fns):
+    """Greatest distance between the unclamped taps of one point."""
+    env = {}
+    for fn in fns:
+        for q in fn.free.collect(C.Parameter):
+            env[q] = 1 << 40
+    at = np.arange(MAX_PERIOD, dtype=np.int64) + (1 << 20)
+    try:
+        v = np.stack([np.broadcast_to(fn.evaluate(at, env, free=True),
+                                      at.shape) for fn in fns])
+    except EvalError:
+        return None
+    return int(np.max(v.max(0) - v.min(0)))
+
+
+def _same_clamps(uses):
+    """Whether every tap is clamped to the same bounds, clamps outermost:
+    the taps of a tile then lie no further apart than without clamps."""
+    keys = set()
+    for t in uses:
+        for fn in t.fns:
+            e, key = fn.expr, []
+            while clamp_arm(e) is not None:
+                arm = clamp_arm(e)
+                key += [(str(b), low) for a, b, low in clamps(e)
+                        if a is arm][:1]
+                e = arm
+            if not key or has_clamp(e):
+                return False
+            keys.add(tuple(key))
+    return len(keys) == 1
+
+
+def _clamped_reads(plan, env, least):
+    """Decide, for every buffer and parametric dimension, how it holds what
+    clamped taps read.  A tile's region follows the unclamped taps (see
+    StencilGen.gen_regions), so that buffers look the same on every tile.
+
+    * The unclamped taps of every point provably enclose its clamped ones
+      (clamps at the producer's edges, at most a tap's offset inside):
+      nothing to do.
+    * Otherwise the region is moved on the tiles that need it
+      (``Node.moved``), provided that it is wide enough: all taps have the
+      same bounds (a crop), or they are the taps of one consumer and the
+      clamps reach past them by a constant that the tile has room for.
+    * Otherwise (``f(max(x, a)) + f(min(x, b))``: a tile's taps may lie
+      anywhere apart) an input is read from HBM, and a stage is not kept in
+      shared memory with its consumers."""
+    for n in plan.nodes:
+        if not n.in_smem:
+            continue
+        for d in range(n.ndims):
+            if _const_extent(n.func.domain[d], env) is not None:
+                continue
+            uses, other = [], False
+            for m in [u[0] for u in n.uses]:
+                if any(m is t.m for t in uses):
+                    continue
+                fns = [fs[d] for q, fs in n.uses if q is m]
+                other = other or any(fn.kind != 'mono' for fn in fns)
+                uses.append(_Taps(m, [fn for fn in fns
+                                      if fn.kind == 'mono'], least))
+            if all(t.inside() for t in uses):
+                continue
+            if n.role != 'out' and not other:
+                if _same_clamps(uses):
+                    n.moved.add(d)
+                    continue
+                if len(uses) == 1 and len(set(
+                        (fn.cdim, fn.dir) for fn in uses[0].fns)) == 1:
+                    reach = uses[0].reach(n.func.domain[d])
+                    wide = _spread(uses[0].fns)
+                    if reach is not None and wide is not None and \
+                            wide + 1 + reach <= n.least_ext[d]:
+                        n.moved.add(d)
+                        continue
+            if n.role != 'stage':
+                raise PlanError("%s: clamped taps too far apart for one "
+                                "tile" % n.name)
+            n.role = 'global'
+            plan.ext_role[n.func] = 'global'
+            n.moved.clear()
+            break
 
 
 def _alignment(plan, env):

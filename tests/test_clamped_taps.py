@@ -69,3 +69,119 @@ def test_clamps_in_a_dimension_of_constant_extent(taps, role, tile,
          tmp_path, tile, "bin_" + taps,
          [('materialize', ['f'])] if role == 'smem' else
          ['inline_budget=100000', 'stage_pointwise'])
+
+
+def _rows(taps, cond=None, lo=0, hi=R - 1):
+    """A filter of two images' rows, the second through shared memory."""
+    img = Image(Float, "img", [R, C])
+    dom = [Interval(Int, lo, hi), Interval(Int, 0, C - 1)]
+    f = Function(([x, y], [Interval(Int, 0, R - 1), dom[1]]), Float, "f")
+    f.defn = [img(x, y) + 1]
+    g = Function(([x, y], dom), Float, "g")
+    e = taps(f)
+    g.defn = [e] if cond is None else [Case(cond, e)]
+    return g
+
+
+def _img(rows, cols):
+    return {'img': np.random.default_rng(rows).random(
+        (rows, cols)).astype(np.float32)}
+
+
+# bounds off the producer's edges by a literal, by a parameter, and taps
+# whose bounds differ; x / 2 and x * 2 with them; indices that run down
+ROW_TAPS = {
+    "literal": (lambda f: f(Min(x + 1, 20), y) + f(Min(x + 2, 20), y), {}),
+    "literals": (lambda f: f(Max(x - 1, 9), y) + f(Min(x + 1, 20), y), {}),
+    "crop": (lambda f: f(Min(Max(x - 1, M), R - 1 - M), y) +
+             f(Min(Max(x + 1, M), R - 1 - M), y), {'M': 8}),
+    "crop_far": (lambda f: f(Min(Max(x - 1, M), R - 1 - M), y) +
+                 f(Min(Max(x + 1, M), R - 1 - M), y), {'M': 30}),
+    "one_sided": (lambda f: f(Max(x - 1, M), y) +
+                  f(Min(x + 1, R - 1 - M), y), {'M': 8}),
+    "one_sided_8": (lambda f: f(Max(x - 1, 8), y) + f(Min(x + 1, R - 9), y),
+                    {}),
+    "one_sided_2": (lambda f: f(Max(x - 1, 2), y) + f(Min(x + 1, R - 3), y),
+                    {}),
+    "edges": (lambda f: f(Max(x - 1, 0), y) + f(Min(x + 1, R - 1), y), {}),
+    "one_tap": (lambda f: f(Max(x - 9, 0), y) + f(Max(x - 8, 0), y), {}),
+    "columns": (lambda f: f(x, Max(y - 3, M)) + f(x, Min(y, C - M)),
+                {'M': 2}),
+    "half": (lambda f: f(Min(Max(x / 2 - 1, M), R - 1), y) +
+             f(Min(x / 2 + 1, R - 1), y), {'M': 3}),
+    "twice": (lambda f: f(Min(2 * x, R - 1 - M), y) +
+              f(Min(2 * x + 1, R - 1 - M), y), {'M': 1}),
+    "down": (lambda f: f(Max(R - 1 - M - x, 0), y) +
+             f(Max(R - 2 - M - x, 0), y), {'M': 3}),
+}
+
+
+@pytest.mark.parametrize("taps", sorted(ROW_TAPS))
+@pytest.mark.parametrize("role", ["smem", "stage"])
+@pytest.mark.parametrize("rows,cols", [(97, 21), (98, 70)])
+def test_clamps_inside_the_domain(taps, role, rows, cols, tmp_path):
+    e, prm = ROW_TAPS[taps]
+    _run(_rows(e), _img(rows, cols), dict(prm, R=rows, C=cols), tmp_path,
+         (16, 32), "row_" + taps,
+         [('materialize', ['f'])] if role == 'smem' else
+         ['inline_budget=100000', 'stage_pointwise'])
+
+
+@pytest.mark.parametrize("taps", ["half", "one_sided_2",
+                                  "edges", "crop", "twice"])
+@pytest.mark.parametrize("tile", [(1, 32), (2, 16), (3, 48)])
+def test_thin_tiles(taps, tile, tmp_path):
+    """Tiles of a few rows: a tap rounded towards zero or clamped easily
+    lies outside what the tile's other taps read."""
+    e, prm = ROW_TAPS[taps]
+    _run(_rows(e), _img(37, 50), dict(prm, R=37, C=50), tmp_path, tile,
+         "thin_" + taps, ['inline_budget=0', 'stage_pointwise'])
+
+
+@pytest.mark.parametrize("opts", [(), ('no_fold_clamps',),
+                                  ('shared_regions',)])
+def test_crops_of_several_stages(opts, tmp_path):
+    """A chain of cropped stages, one of them an output too, and a second
+    consumer with the same crop."""
+    def crop(v, hi):
+        return Min(Max(v, M), hi - 1 - M)
+    img = Image(Float, "img", [R, C])
+    dom = [Interval(Int, 0, R - 1), Interval(Int, 0, C - 1)]
+    fs = []
+    for n in "fgh":
+        fs.append(Function(([x, y], dom), Float, n))
+    f, g, h = fs
+    f.defn = [img(crop(x - 1, R), y) + img(crop(x + 1, R), crop(y, C))]
+    g.defn = [Case(Condition(x, ">=", 3), f(crop(x + 2, R), y) +
+                   f(crop(x - 2, R), y))]
+    h.defn = [g(x, crop(y - 1, C)) + g(x, crop(y + 1, C)) +
+              f(crop(x, R), y)]
+    prm = {'R': 45, 'C': 71, 'M': 6}
+    inputs = _img(45, 71)
+    for outs in ([h], [h, g]):
+        p = buildPipeline(outs, param_estimates=[(R, 500), (C, 500), (M, 6)],
+                          tile_sizes=[8, 16], pipe_name="crops%d" % len(outs),
+                          options=['inline_budget=0'] + list(opts))
+        got = emulate.run(p, prm, inputs, tmp_path, fill=0)
+        ev = Evaluator(prm, inputs)
+        for o in outs:
+            # float32 sums of at most ten values below 1
+            assert np.abs(got[o.name] - ev.array(o)).max() <= \
+                10 * 16 * 2.0 ** -24
+
+
+def test_edge_clamps_keep_their_stages():
+    """Clamps at the producer's edges, or at most a tap's offset inside
+    them, move no region; a crop moves it; taps that may lie anywhere apart
+    keep a stage out of the tile."""
+    for taps, moved in (("edges", False), ("literal", True),
+                        ("crop", True), ("one_sided_8", True),
+                        ("one_sided", None), ("literals", None)):
+        e, prm = ROW_TAPS[taps]
+        p = buildPipeline(
+            [_rows(e)], param_estimates=[(R, 500), (C, 500)] +
+            ([(M, 8)] if prm else []), tile_sizes=[16, 32],
+            pipe_name="keep_" + taps, options=['inline_budget=0'])
+        n = [n for q in p.groups for n in q.plan.nodes if n.name == "f" and
+             n.role != 'out']
+        assert [bool(q.moved) if q.in_smem else None for q in n] == [moved]
