@@ -2383,6 +2383,8 @@ class StencilGen(object):
                                  for b in mb[fn.cdim]]
                             if fn.dir < 0:
                                 t.reverse()
+                            if fn.up and not self.const_dim(n.func, d):
+                                t[1] = "(%s + %d)" % (t[1], fn.up)
                         elif fn.kind == 'const':
                             t = [ctx.expr(fn.expr, {})] * 2
                         else:

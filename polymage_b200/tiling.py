@@ -55,7 +55,7 @@ from .expression import substitute_vars
 from .evaluate import (is_min_max, eval_int, EvalError, monotone_dir, divisors_in,
                        clamps, clamp_arm, has_clamp, strip_clamps,
                        try_eval_int, _has_loop_var)
-from .bounds import AtEnd, at_most, excess, least_params
+from .bounds import AtEnd, at_most, excess, least_params, not_negative
 
 SMEM_BUDGET = 200 * 1024       # bytes per CTA we allow a plan to use
 DEFAULT_THREADS = 256
@@ -84,6 +84,9 @@ class IndexFn(object):
         # (see bind_clamps)
         self.free = self.expr
         self.clamped = self.whole = False
+        # how far above the rounded-down index a quotient rounded towards
+        # zero can lie (see _rounded)
+        self.up = 0
         e = self.expr
         if is_data_dependent(e):
             return
@@ -605,6 +608,11 @@ def plan_stencil(pipeline, comps, tile=None):
         # materialized consumers read only where their Case holds
         n.case_box = case_box(n.func) if n.role in ('out', 'smem') else None
     least = least_params(pipeline)
+    for n in nodes:
+        for m, fns in n.uses:
+            for fn in fns:
+                if fn.kind == 'mono':
+                    fn.up = _rounded(fn, m, least)
     plan.nodes = nodes
     plan.node_of = node_of
 
@@ -815,6 +823,8 @@ def infer_regions(plan, anchor_box, env, clamp=True, tile_first=None):
                     a = fn.evaluate(mlo[fn.cdim], env, not fixed[d])
                     b = fn.evaluate(mhi[fn.cdim], env, not fixed[d])
                     a, b = np.minimum(a, b), np.maximum(a, b)
+                    if not fixed[d]:
+                        b = b + fn.up
                 elif fn.kind == 'const':
                     a = b = fn.evaluate(0, env)
                 else:
@@ -988,6 +998,27 @@ def _bound_forms(e, sign=1):
     return None if has_clamp(e) else []
 
 
+def _rounded(fn, m, least):
+    """Divisions of index ``fn`` whose numerator may be negative at a point
+    of consumer ``m``: regions round them down, the tap rounds towards
+    zero."""
+    cb = getattr(m, 'case_box', None)
+    lows = [m.func.domain[fn.cdim].lowerBound] + (
+        list(cb[fn.cdim][0]) if cb else [])
+    out = 0
+    stack = [fn.free]
+    while stack:
+        e = stack.pop()
+        if isinstance(e, AbstractBinaryOpNode):
+            if e.op == '/' and _has_loop_var(e.left) and not any(
+                    not_negative(e.left, fn.var, q, least) for q in lows):
+                out += 1
+            stack += [e.left, e.right]
+        elif isinstance(e, AbstractUnaryOpNode):
+            stack.append(e.child)
+    return out
+
+
 class _Taps(object):
     """The taps of one consumer into one parametric dimension."""
 
@@ -1070,7 +1101,7 @@ def _spread(fns):
                                       at.shape) for fn in fns])
     except EvalError:
         return None
-    return int(np.max(v.max(0) - v.min(0)))
+    return int(np.max(v.max(0) - v.min(0))) + max(fn.up for fn in fns)
 
 
 def _same_clamps(uses):

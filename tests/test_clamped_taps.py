@@ -113,6 +113,8 @@ ROW_TAPS = {
               f(Min(2 * x + 1, R - 1 - M), y), {'M': 1}),
     "down": (lambda f: f(Max(R - 1 - M - x, 0), y) +
              f(Max(R - 2 - M - x, 0), y), {'M': 3}),
+    "quotient": (lambda f: f(Max((x - 3) / 2, 0), y) +
+                 f(Max((x - 1) / 2, 0), y), {}),
 }
 
 
@@ -127,7 +129,7 @@ def test_clamps_inside_the_domain(taps, role, rows, cols, tmp_path):
          ['inline_budget=100000', 'stage_pointwise'])
 
 
-@pytest.mark.parametrize("taps", ["half", "one_sided_2",
+@pytest.mark.parametrize("taps", ["quotient", "half", "one_sided_2",
                                   "edges", "crop", "twice"])
 @pytest.mark.parametrize("tile", [(1, 32), (2, 16), (3, 48)])
 def test_thin_tiles(taps, tile, tmp_path):
@@ -136,6 +138,28 @@ def test_thin_tiles(taps, tile, tmp_path):
     e, prm = ROW_TAPS[taps]
     _run(_rows(e), _img(37, 50), dict(prm, R=37, C=50), tmp_path, tile,
          "thin_" + taps, ['inline_budget=0', 'stage_pointwise'])
+
+
+def test_negative_numerators_without_a_clamp(tmp_path):
+    """(x - 3) / 2 at x = 2 is 0, which rounding down would miss."""
+    g = _rows(lambda f: f((x - 3) / 2, y) + f((x - 3) / 2, Max(y - 1, 0)),
+              lo=2)
+    for tile in ((1, 32), (4, 16)):
+        _run(g, _img(21, 40), {'R': 21, 'C': 40}, tmp_path, tile,
+             "negative%d" % tile[0], ['inline_budget=0', 'stage_pointwise'])
+
+
+def test_negative_domains(tmp_path):
+    """Tiles whose numerators are all negative."""
+    img = Image(Float, "img", [R, C])
+    cols = Interval(Int, 0, C - 1)
+    f = Function(([x, y], [Interval(Int, -20, R - 21), cols]), Float, "f")
+    f.defn = [img(x + 20, y) + 1]
+    g = Function(([x, y], [Interval(Int, 0, 2 * R - 50), cols]), Float, "g")
+    g.defn = [f((x - 35) / 2, y) + f((x - 35) / 2, Max(y - 1, 0))]
+    for tile in ((4, 32), (3, 16)):
+        _run(g, _img(33, 40), {'R': 33, 'C': 40}, tmp_path, tile,
+             "negdom%d" % tile[0], ['inline_budget=0', 'stage_pointwise'])
 
 
 @pytest.mark.parametrize("opts", [(), ('no_fold_clamps',),
