@@ -2011,7 +2011,7 @@ class StencilGen(object):
             if id(n.func) not in seen:
                 seen.add(id(n.func))
                 pg.declare_domain(w, n.func, self.ctx, False)
-        self.gen_regions()
+        self.gen_regions(host=True)
         w("(void)t0;")
         for j, f in enumerate(pg.inputs):
             w("in_end[%d] = 0;" % j)
@@ -2023,10 +2023,11 @@ class StencilGen(object):
             nd = n.ndims
             w.open("")
             empty = []
+            r = "n" if self.clamped_global(n) else "r"
             for d in range(nd):
-                w("const int h%d = pm_imin(r_%s_hi%d, d_%s_hi%d), l%d = "
-                  "pm_imax(r_%s_lo%d, d_%s_lo%d);" % (d, nm, d, fnm, d, d, nm,
-                                                      d, fnm, d))
+                w("const int h%d = pm_imin(%s_%s_hi%d, d_%s_hi%d), l%d = "
+                  "pm_imax(%s_%s_lo%d, d_%s_lo%d);" % (
+                      d, r, nm, d, fnm, d, d, r, nm, d, fnm, d))
                 empty.append("l%d > h%d" % (d, d))
             w("long long o = 0, s = 1;")
             for d in range(nd - 1, -1, -1):
@@ -2329,7 +2330,14 @@ class StencilGen(object):
                     hi = "pm_imin(%s, %d)" % (hi, _const_int(e))
         return lo, hi
 
-    def gen_regions(self):
+    def clamped_global(self, n):
+        """Whether a node is read from HBM through clamped taps: its region
+        follows the unclamped ones and need not hold what they read."""
+        return n.role == 'global' and any(
+            fn.kind == 'mono' and fn.clamped
+            for _, fns in n.uses for fn in fns)
+
+    def gen_regions(self, host=False):
         """The region of every node for the tile: ``r_<node>_lo/hi``.
 
         Regions are not clamped to the image: along a parametric dimension
@@ -2349,6 +2357,8 @@ class StencilGen(object):
         big = "0x3fffffff"
         ctx.floor_div = True
         self.shifts = []
+        reads = any(n.moved or host and self.clamped_global(n)
+                    for n in plan.nodes)
         for n in plan.nodes:
             nm = self.node_name(n)
             fnm = pg.fn(n.func)
@@ -2433,8 +2443,8 @@ class StencilGen(object):
                     if self.const_dim(n.func, d):
                         w("r_%s_lo%d = %s; r_%s_hi%d = %s;" % (
                             nm, d, lo, nm, d, hi))
-            if any(q.moved for q in plan.nodes) and (n.in_smem or
-                                                     n.role == 'out'):
+            if reads and (n.in_smem or n.role == 'out' or
+                          host and self.clamped_global(n)):
                 ctx.floor_div = False
                 self.gen_reads(n)
                 ctx.floor_div = True

@@ -4,6 +4,9 @@ bounds of a clamp are not the edges of the producer's domain.  Kernels run
 on the CPU (tests/emulate.py) against the point-by-point evaluation of the
 definitions; shared memory that no loop or copy wrote reads as NaN."""
 
+import ctypes
+import subprocess
+
 import numpy as np
 import pytest
 
@@ -209,3 +212,49 @@ def test_edge_clamps_keep_their_stages():
         n = [n for q in p.groups for n in q.plan.nodes if n.name == "f" and
              n.role != 'out']
         assert [bool(q.moved) if q.in_smem else None for q in n] == [moved]
+
+
+@pytest.mark.parametrize("opts", [('no_stage',), ('stage_pointwise',)])
+@pytest.mark.parametrize("crop", [0, 5, 60])
+def test_bands_copy_what_their_tiles_read(opts, crop, tmp_path):
+    """The host entry copies a prefix of each input before a band of tiles
+    runs: the footprint function has to cover the clamped rows, also those
+    far from the band."""
+    img = Image(Float, "img", [R, C])
+    g = Function(([x, y], [Interval(Int, 0, R - 1), Interval(
+        Int, 0, C - 1)]), Float, "g")
+
+    def at(v):
+        return img(Min(Max(v, M), R - 1 - M), y)
+    g.defn = [at(x - 1) + at(x + 1)]
+    p = buildPipeline([g], param_estimates=[(R, 500), (C, 500), (M, 5)],
+                      tile_sizes=[16, 32], pipe_name="bands%d" % crop,
+                      options=list(opts))
+    src = p.generate_code().source
+    k = "pm_bands%d_g0" % crop
+    body = src[src.index("static void %s_footprint(" % k):]
+    body = body[body.index("{") + 1:body.index("\n}\n")]
+    rows, cols = 150, 40
+    (tmp_path / "fp.cpp").write_text("""
+static int pm_imin(int a, int b) { return a < b ? a : b; }
+static int pm_imax(int a, int b) { return a > b ? a : b; }
+static int pm_floordiv(int a, int b) { int q = a / b; return (q * b != a &&
+  ((a < 0) != (b < 0))) ? q - 1 : q; }
+struct D_t { int p_R, p_C, p_M, glo[2], ghi[2], gn[2], tile_base; };
+extern "C" void fp(const D_t* Dp, int tile, long long* in_end, int* a_lo,
+                   int* a_hi) { const D_t& D = *Dp;
+""" + body + "}\n")
+    so = str(tmp_path / "fp.so")
+    subprocess.run(["g++", "-O1", "-w", "-shared", "-fPIC",
+                    str(tmp_path / "fp.cpp"), "-o", so], check=True)
+    D = (ctypes.c_int * 10)(rows, cols, crop, 0, 0, rows - 1, cols - 1,
+                            -(-rows // 16), -(-cols // 32), 0)
+    end = (ctypes.c_longlong * 1)()
+    lo, hi = (ctypes.c_int * 2)(), (ctypes.c_int * 2)()
+    lib = ctypes.CDLL(so)
+    for tile in range(D[7] * D[8]):
+        lib.fp(D, tile, end, lo, hi)
+        last = min(lo[0] + 15, rows - 1)
+        need = max(min(max(v, crop), rows - 1 - crop)
+                   for q in (lo[0], last) for v in (q - 1, q + 1))
+        assert end[0] >= need * cols + hi[1] + 1, (tile, lo[0], end[0])
