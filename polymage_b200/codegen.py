@@ -583,6 +583,17 @@ def _clamp_arm(e):
     return None if is_data_dependent(e) else clamp_arm(e)
 
 
+def _typed_text(e):
+    """Text of arithmetic on parameters and literals with their types."""
+    e = Value.numericToValue(e)
+    if isinstance(e, AbstractBinaryOpNode):
+        return "(%s %s %s)" % (_typed_text(e.left), e.op,
+                               _typed_text(e.right))
+    if isinstance(e, AbstractUnaryOpNode):
+        return "(%s%s)" % (e.op, _typed_text(e.child))
+    return "%s:%s" % (e, e.typ.c_type_name())
+
+
 def _uniform_quotient(e):
     """Whether ``e`` is floating-point arithmetic on parameters and
     literals with a division in it."""
@@ -1973,7 +1984,8 @@ class StencilGen(object):
         self.gen_footprint()
 
     def hoist(self, e):
-        key = str(e)
+        # (a float and a double literal print alike)
+        key = _typed_text(e)
         if key not in self.hoisted:
             t = "double" if getType(e) is C.Double else "float"
             self.hoisted[key] = (t, "h_%d" % len(self.hoisted), e)
