@@ -596,7 +596,8 @@ def _typed_text(e):
 
 def _uniform_quotient(e):
     """Whether ``e`` is floating-point arithmetic on parameters and
-    literals with a division in it."""
+    literals with a division in it, and without a division of integers:
+    evaluated ahead of any Case, on the host, one by zero would trap."""
     def ok(x):
         """(arithmetic on parameters and literals, divides floats)"""
         x = Value.numericToValue(x)
@@ -606,9 +607,10 @@ def _uniform_quotient(e):
             return ok(x.child)
         if isinstance(x, AbstractBinaryOpNode) and x.op in '+-*/':
             a, b = ok(x.left), ok(x.right)
-            return a[0] and b[0], a[1] or b[1] or (
-                x.op == '/' and a[0] and b[0] and
-                getType(x) in (C.Float, C.Double))
+            if not (a[0] and b[0]):
+                return False, False
+            divides = x.op == '/' and getType(x) in (C.Float, C.Double)
+            return x.op != '/' or divides, a[1] or b[1] or divides
         return False, False
     return ok(e) == (True, True)
 

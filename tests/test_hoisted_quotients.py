@@ -1,15 +1,16 @@
 """Quotients of parameters that a launch carries precomputed: computed in
-their own precision."""
+their own precision, and none whose evaluation on the host could trap."""
 
 import numpy as np
 
 from polymage_b200.compiler import buildPipeline
-from polymage_b200.constructs import (Double, Float, Function, Image,
-                                      Int, Interval, Parameter, Variable)
+from polymage_b200.constructs import (Case, Condition, Double, Float,
+                                      Function, Image, Int, Interval,
+                                      Parameter, Variable)
 from polymage_b200.expr_ast import Value
 from tests import emulate
 
-R, C = Parameter(Int, "R"), Parameter(Int, "C")
+R, C, N, M = (Parameter(Int, n) for n in "RCNM")
 h = Parameter(Float, "h")
 x, y = Variable(Int, "x"), Variable(Int, "y")
 DOM = [Interval(Int, 0, R - 1), Interval(Int, 0, C - 1)]
@@ -34,6 +35,21 @@ def test_equal_texts_of_different_precision(tmp_path):
     one, third = np.float64(np.float32(1) / np.float32(3)), 1 / 3.0
     # float64 rounding of four operations
     assert np.abs(got - (img * one + img * third * 3)).max() <= 4 * 2.0 ** -52
+
+
+def test_integer_quotients_stay_in_their_case(tmp_path):
+    """1.0 / (N / M) with M = 0 under a Case that does not hold."""
+    p = _build(Float, lambda img: [
+        Case(Condition(M, ">", 0), img(x, y) * (1.0 / (N / M))),
+        Case(Condition(M, "<=", 0), img(x, y) + 2)], "quot_int",
+        (N, 6), (M, 2))
+    src = p.generate_code().source
+    assert "h_0" not in src
+    img = np.random.default_rng(2).random((9, 40)).astype(np.float32)
+    for m, want in ((2, img / 3), (0, img + 2)):
+        got = emulate.run(p, {'R': 9, 'C': 40, 'N': 6, 'M': m},
+                          {'img': img}, tmp_path)["g"]
+        assert np.abs(got - want).max() <= 2 * 2.0 ** -23
 
 
 def test_the_solvers_quotients_are_still_precomputed():
