@@ -2317,13 +2317,13 @@ class StencilGen(object):
                            for d in range(n.ndims))
 
     def const_dim(self, f, d):
-        """Whether dimension ``d`` of ``f`` has an extent free of
+        """Whether dimension ``d`` of ``f`` lies at a place free of
         parameters (channels, a grid's intensity bins)."""
-        from .tiling import _const_extent
+        from .tiling import _fixed_extent
         key = (id(f), d)
         memo = self.pg.__dict__.setdefault('_const_dims', {})
         if key not in memo:
-            memo[key] = _const_extent(f.domain[d],
+            memo[key] = _fixed_extent(f.domain[d],
                                       self.pg.p.int_env()) is not None
         return memo[key]
 

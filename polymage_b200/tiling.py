@@ -113,8 +113,8 @@ class IndexFn(object):
         and hold exactly what the clamped index takes.  That needs the
         consumer's dimension to be of constant extent too and bounds that
         are literals; otherwise the region is the whole dimension."""
-        if self.clamped and _const_extent(dom, env) is not None:
-            self.whole = _const_extent(consumer_dom, env) is None or any(
+        if self.clamped and _fixed_extent(dom, env) is not None:
+            self.whole = _fixed_extent(consumer_dom, env) is None or any(
                 b.collect(C.Parameter) for _, b, _ in clamps(self.expr))
 
     def evaluate(self, value, env, free=False):
@@ -716,6 +716,16 @@ def _const_extent(dom, env):
     return a
 
 
+def _fixed_extent(dom, env):
+    """Extent of an interval whose bounds are numbers, so that it lies at
+    the same place in every image; None for others (also ``[R, R + 5]``:
+    regions there are inferred as along any parametric dimension)."""
+    if try_eval_int(dom.lowerBound, {}) is None or \
+            try_eval_int(dom.upperBound, {}) is None:
+        return None
+    return _const_extent(dom, env)
+
+
 def _domain_vals(func, env):
     out = []
     for d in func.domain:
@@ -753,7 +763,7 @@ def case_restricted(node, region, env, constant_only=False):
     hi = list(hi)
     env2 = dict((k, v * 3 + 17) for k, v in env.items())
     for d, (los, his) in enumerate(cb):
-        if constant_only and _const_extent(node.func.domain[d], env) is None:
+        if constant_only and _fixed_extent(node.func.domain[d], env) is None:
             continue
         for e in los:
             v = try_eval_int(e, env)
@@ -808,7 +818,7 @@ def infer_regions(plan, anchor_box, env, clamp=True, tile_first=None):
             hi = [np.minimum(h, dom[d][1]) for d, h in enumerate(hi)]
         # unclamped, the image is taken to have no borders: only the
         # dimensions of constant extent keep theirs
-        fixed = [clamp or _const_extent(q, env) is not None
+        fixed = [clamp or _fixed_extent(q, env) is not None
                  for q in n.func.domain]
         for m, fns in n.uses:
             mlo, mhi = case_restricted(m, regions[m.func], env,
@@ -900,7 +910,7 @@ def _static_extents(plan, env):
         # starts at a constant, when only glo + j*tile occur
         axes = []
         for k, t in enumerate(plan.tile):
-            if _const_extent(plan.anchor.domain[k], env) is not None:
+            if _fixed_extent(plan.anchor.domain[k], env) is not None:
                 lo0, hi0 = adom[k]
                 axes.append(np.arange(lo0, hi0 + 1, t, dtype=np.int64))
             elif glo[k] is not None:
@@ -914,7 +924,7 @@ def _static_extents(plan, env):
         for k, t in enumerate(plan.tile):
             lo = grids[k].ravel()
             hi = lo + t - 1
-            if _const_extent(plan.anchor.domain[k], env) is not None:
+            if _fixed_extent(plan.anchor.domain[k], env) is not None:
                 hi = np.minimum(hi, adom[k][1])
             box.append((lo, hi))
         regs = infer_regions(plan, box, env, clamp=False)
@@ -940,7 +950,7 @@ def _static_extents(plan, env):
             n.const_bounds = dict(
                 (d, (np.asarray(lo[d]), np.asarray(hi[d])))
                 for d in range(n.ndims)
-                if _const_extent(n.func.domain[d], env) is not None)
+                if _fixed_extent(n.func.domain[d], env) is not None)
         exts.append(cur)
     for n in plan.nodes:
         a, b = exts[0][n.func], exts[1][n.func]
@@ -1141,7 +1151,7 @@ def _clamped_reads(plan, env, least):
         if not n.in_smem:
             continue
         for d in range(n.ndims):
-            if _const_extent(n.func.domain[d], env) is not None:
+            if _fixed_extent(n.func.domain[d], env) is not None:
                 continue
             uses, other = [], False
             for m in [u[0] for u in n.uses]:
@@ -1198,7 +1208,7 @@ def _alignment(plan, env):
         for m, fns in n.uses:
             for d, fn in enumerate(fns):
                 if fn.kind != 'mono' or m.align[fn.cdim] is None or \
-                        fn.clamped and _const_extent(n.func.domain[d],
+                        fn.clamped and _fixed_extent(n.func.domain[d],
                                                      env) is not None:
                     continue
                 try:
@@ -1276,7 +1286,7 @@ def _layout_smem(plan, tight=False, env=None, prefetch=False,
             not no_pairs
         if n.role == 'stage':
             al = max(1, 16 // es)
-            whole = env is not None and _const_extent(
+            whole = env is not None and _fixed_extent(
                 n.func.domain[-1], env) == ext[-1]
             if tight and whole and ext[-1] < al:
                 w = ext[-1]

@@ -1,0 +1,53 @@
+"""Dimensions of constant extent that lie at a place given by parameters
+(``[R, R + 5]``): tiles, regions and buffers follow the parameters of the
+call.  Kernels run on the CPU against the definitions."""
+
+import numpy as np
+import pytest
+
+from polymage_b200.compiler import buildPipeline
+from polymage_b200.constructs import (Case, Condition, Float, Function,
+                                      Image, Int, Interval, Max, Parameter,
+                                      Variable)
+from tests import emulate
+from tests.dsl_eval import Evaluator
+
+R, C = Parameter(Int, "R"), Parameter(Int, "C")
+x, y = Variable(Int, "x"), Variable(Int, "y")
+PLACED, COLS = Interval(Int, R, R + 5), Interval(Int, 0, C - 1)
+
+
+def _outer(img):
+    f = Function(([x, y], [PLACED, COLS]), Float, "f")
+    f.defn = [img(x - R, y) + 1]
+    g = Function(([x, y], [PLACED, COLS]), Float, "g")
+    g.defn = [Case(Condition(x, "<=", R + 4), f(x, y) + f(x + 1, Max(
+        y - 1, 0)) + f(x, Max(y - 2, 0)))]
+    return g
+
+
+def _inner(img):
+    f = Function(([y, x], [COLS, PLACED]), Float, "f")
+    f.defn = [img(x - R, y) + 1]
+    g = Function(([y, x], [COLS, PLACED]), Float, "g")
+    g.defn = [f(y, x) + f(Max(y - 1, 0), R + 1) + f(Max(y - 2, 0), R)]
+    return g
+
+
+@pytest.mark.parametrize("defn", [_outer, _inner])
+@pytest.mark.parametrize("opts", [('inline_budget=0',),
+                                  ('inline_budget=100000',),
+                                  ('inline_budget=0', ('materialize',
+                                                       ['f']))])
+@pytest.mark.parametrize("rows", [0, 1, 21])
+def test_values_at_their_place(defn, opts, rows, tmp_path):
+    g = defn(Image(Float, "img", [6, C]))
+    p = buildPipeline([g], param_estimates=[(R, 500), (C, 500)],
+                      tile_sizes=[4, 16], pipe_name="placed" +
+                      defn.__name__, options=list(opts))
+    img = np.random.default_rng(rows).random((6, 45)).astype(np.float32)
+    prm = {'R': rows, 'C': 45}
+    got = emulate.run(p, prm, {'img': img}, tmp_path, fill=0)["g"]
+    ref = Evaluator(prm, {'img': img}).array(g)
+    # float32 sums of three values below 2
+    assert np.abs(got - ref).max() <= 4 * 8 * 2.0 ** -24
