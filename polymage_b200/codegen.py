@@ -725,6 +725,19 @@ def _subst(a, bind):
     return substitute_vars(a, m)
 
 
+def _split_cond(cond, tbind):
+    """Conjuncts of a condition, those that read data (themselves or in a
+    target index that stands for a function variable) apart."""
+    if cond.conditional == '&&':
+        a, b = _split_cond(cond.lhs, tbind), _split_cond(cond.rhs, tbind)
+        return a[0] + b[0], a[1] + b[1]
+    reads = cond.has(C.Reference) or any(
+        hasattr(tbind.get(v), 'has') and (
+            isinstance(tbind[v], C.Reference) or tbind[v].has(C.Reference))
+        for v in cond.collect(C.Variable))
+    return ([], [cond]) if reads else ([cond], [])
+
+
 def tbind_of(f, rvars, red, rbind):
     """Binding for a reduction part: reduction variables to the loop
     variables, and every other function variable to the part's target
@@ -4468,10 +4481,10 @@ class ReductionGen(object):
             # point of the reduction domain (checked per call), so they
             # share one scope: values they have in common (e.g. an input
             # pixel) are read once.
+            # The others' reads, those of a data-dependent target among
+            # them, are in bounds only where the condition holds.
             shared = cond is None or _cond_const_true(cond, tbind)
-            if not shared:
-                ctx.push()
-                w.open("")
+            then = ["pm_pt"] if shared else self.open_part(ctx, cond, tbind)
             tgt = red.accumulate_ref.arguments
             cn = ["c%d_%d" % (d, pi) for d in range(nd)]
             for d, ta in enumerate(tgt):
@@ -4479,12 +4492,11 @@ class ReductionGen(object):
             # target coordinates that do not depend on data are inside
             # the domain wherever the call passed the bounds validation;
             # only data-dependent ones (a bin index) are tested
-            inb = " && ".join("%s >= d_%s_lo%d && %s <= d_%s_hi%d" % (
+            inb = ["%s >= d_%s_lo%d && %s <= d_%s_hi%d" % (
                 cn[d], fnm, d, cn[d], fnm, d) for d in range(nd)
-                if is_data_dependent(tgt[d])) or "true"
-            cc = ctx.cond(cond, tbind) if cond is not None else "true"
+                if is_data_dependent(tgt[d])]
             val = ctx.expr(expr, rbind) if shared else None
-            w.open("if (pm_pt && (%s) && (%s))" % (inb, cc))
+            w.open("if (%s)" % (" && ".join(then + inb) or "true"))
             if val is None:
                 val = ctx.expr(expr, rbind)
             if priv:
@@ -4547,6 +4559,15 @@ class ReductionGen(object):
         E = plan.tile[-1]
         return k if k > 1 and E % k == 0 and E // k >= 32 else 0
 
+    def open_part(self, ctx, cond, tbind):
+        """Open the scope of a part whose condition decides what it reads:
+        what reads data in the condition comes after the rest of it."""
+        ctx.push()
+        first, then = _split_cond(cond, tbind)
+        self.pg.w.open("if (%s)" % " && ".join(
+            ["pm_pt"] + [ctx.cond(c, tbind) for c in first]))
+        return [ctx.cond(c, tbind) for c in then]
+
     def gen_cells(self, ctx, parts):
         """Grid-cell form (tiling._cell_map): a thread owns one column of
         points and walks it a cell's rows at a time, adding into bins of
@@ -4601,9 +4622,7 @@ class ReductionGen(object):
         for cond, expr, red in parts:
             tbind = tbind_of(f, rvars, red, rbind)
             shared = cond is None or _cond_const_true(cond, tbind)
-            if not shared:
-                ctx.push()
-                w.open("")
+            then = ["pm_pt"] if shared else self.open_part(ctx, cond, tbind)
             tgt = red.accumulate_ref.arguments
             at, inb = [], []
             for d, st in sorted(strides.items()):
@@ -4613,9 +4632,8 @@ class ReductionGen(object):
                 at.append("%s * %d" % (c, st * nt))
                 if is_data_dependent(tgt[d]):
                     inb.append("(unsigned)%s < %du" % (c, bins[d]))
-            cc = ctx.cond(cond, tbind) if cond is not None else "true"
             val = ctx.expr(expr, rbind) if shared else None
-            w.open("if (%s)" % " && ".join(["pm_pt"] + inb + [cc]))
+            w.open("if (%s)" % (" && ".join(then + inb) or "true"))
             if val is None:
                 val = ctx.expr(expr, rbind)
             w("acc[%s] += (%s)(%s);" % (" + ".join(at + ["(int)threadIdx.x"]),

@@ -1,0 +1,53 @@
+"""Sums whose parts read under a condition: the pixel that gives a value or
+a bin may lie outside the image where the condition does not hold.  Every
+form of the sum runs on the CPU, which refuses reads outside a buffer."""
+
+import numpy as np
+import pytest
+
+from polymage_b200.compiler import buildPipeline
+from polymage_b200.constructs import (Case, Cast, Condition, Float, Function,
+                                      Image, Int, Interval, Op, Parameter,
+                                      Reduce, Reduction, Variable)
+from tests import emulate
+
+R, C = Parameter(Int, "R"), Parameter(Int, "C")
+x, y, i, j, b = (Variable(Int, n) for n in "xyijb")
+BINS = 6
+
+
+@pytest.mark.parametrize("form,k,opts", [
+    ("cells", 8, ()), ("privatized", 8, ('no_cells',)),
+    ("atomics", 8, ('no_cells', 'no_privatize')), ("other cells", 5, ())])
+@pytest.mark.parametrize("bins", ["all", "low"])
+def test_reads_stay_under_their_condition(form, k, opts, bins, tmp_path):
+    img, idx = Image(Float, "img", [R, C]), Image(Int, "idx", [R, C])
+    dom = [Interval(Int, 0, R / k + 1), Interval(Int, 0, C / 8 + 1),
+           Interval(Int, 0, BINS - 1)]
+    h = Reduction(([i, j, b], dom), ([x, y], [
+        Interval(Int, 0, R - 1), Interval(Int, 0, C - 1)]), Float, "h")
+    cond = Condition(x, "<=", R - 2) & Condition(y, ">=", 1)
+    if bins == "low":
+        cond = cond & Condition(b, "<=", 2)
+    h.defn = [Case(cond, Reduce(h(x / k, y / 8, Cast(Int, idx(x + 1, y - 1))),
+                                img(x + 1, y - 1), Op.Sum))]
+    h.default = 0
+    g = Function(([i, j, b], dom), Float, "g")
+    g.defn = [h(i, j, b) + 1]
+    p = buildPipeline([g], param_estimates=[(R, 500), (C, 500)],
+                      tile_sizes=[16, 64], pipe_name="cond_red",
+                      options=list(opts))
+    rows, cols = 21, 45
+    rng = np.random.default_rng(k)
+    inputs = {'img': rng.random((rows, cols)).astype(np.float32),
+              'idx': rng.integers(-1, BINS + 1, (rows, cols)).astype(
+                  np.int32)}
+    got = emulate.run(p, {'R': rows, 'C': cols}, inputs, tmp_path)["g"]
+    ref = np.ones(got.shape)
+    X, Y = np.mgrid[0:rows - 1, 1:cols]
+    z = inputs['idx'][1:, :-1]
+    ok = (z >= 0) & (z < (3 if bins == "low" else BINS))
+    np.add.at(ref, (X[ok] // k, Y[ok] // 8, z[ok]),
+              inputs['img'][1:, :-1][ok].astype(np.float64))
+    # float32 sums of at most 64 values below 1
+    assert np.abs(got - ref).max() <= 64 * 64 * 2.0 ** -24
