@@ -1491,13 +1491,21 @@ def plan_reduction(pipeline, comps):
         hi = np.full(period, -(1 << 60))
         for fns in fns_all:
             fn = fns[d]
-            if fn.kind == 'mono':
+            kind = fn.kind
+            if fn.clamped and kind == 'mono':
+                # the tile's clamped targets lie no further apart than the
+                # unclamped ones if there is one clamp only; anywhere in
+                # the dimension else
+                if _const_extent(f.domain[d], env) is not None or \
+                        len(set(q[d].key() for q in fns_all)) > 1:
+                    kind = 'full'
+            if kind == 'mono':
                 t = plan.tile[fn.cdim]
-                a = fn.evaluate(base + r, env)
-                b = fn.evaluate(base + r + t - 1, env)
+                a = fn.evaluate(base + r, env, free=True)
+                b = fn.evaluate(base + r + t - 1, env, free=True)
                 lo = np.minimum(lo, np.minimum(a, b))
                 hi = np.maximum(hi, np.maximum(a, b))
-            elif fn.kind == 'const':
+            elif kind == 'const':
                 v = fn.evaluate(0, env)
                 lo = np.minimum(lo, v)
                 hi = np.maximum(hi, v)

@@ -7,9 +7,11 @@ import pytest
 
 from polymage_b200.compiler import buildPipeline
 from polymage_b200.constructs import (Case, Cast, Condition, Float, Function,
-                                      Image, Int, Interval, Op, Parameter,
-                                      Reduce, Reduction, Variable)
+                                      Image, Int, Interval, Max, Min, Op,
+                                      Parameter, Reduce, Reduction,
+                                      Variable)
 from tests import emulate
+from tests.dsl_eval import Evaluator
 
 R, C = Parameter(Int, "R"), Parameter(Int, "C")
 x, y, i, j, b = (Variable(Int, n) for n in "xyijb")
@@ -51,3 +53,37 @@ def test_reads_stay_under_their_condition(form, k, opts, bins, tmp_path):
               inputs['img'][1:, :-1][ok].astype(np.float64))
     # float32 sums of at most 64 values below 1
     assert np.abs(got - ref).max() <= 64 * 64 * 2.0 ** -24
+
+
+TARGETS = {
+    "row bin": lambda v, w: (v / 8, w / 8, Min(v / 8, 3)),
+    "low rows": lambda v, w: (Min(v / 8, 1), w / 8, 2),
+    "last row": lambda v, w: (Min(v / 5, R / 8), w / 8, 2),
+    "first rows": lambda v, w: (Max(v / 8 - 1, 0), w / 8, 2),
+}
+
+
+@pytest.mark.parametrize("target", sorted(TARGETS))
+@pytest.mark.parametrize("opts", [(), ('no_privatize',)])
+def test_clamped_targets(target, opts, tmp_path):
+    """Targets with a clamped index: a tile near the clamp adds into more
+    cells than one far from it."""
+    img = Image(Float, "img", [R, C])
+    dom = [Interval(Int, 0, R / 8 + 1), Interval(Int, 0, C / 8 + 1),
+           Interval(Int, 0, BINS - 1)]
+    h = Reduction(([i, j, b], dom), ([x, y], [
+        Interval(Int, 0, R - 1), Interval(Int, 0, C - 1)]), Float, "h")
+    h.defn = [Reduce(h(*TARGETS[target](x, y)), img(x, y), Op.Sum)]
+    h.default = 0
+    g = Function(([i, j, b], dom), Float, "g")
+    g.defn = [h(i, j, b) + 1]
+    p = buildPipeline([g], param_estimates=[(R, 30), (C, 500)],
+                      tile_sizes=[16, 64], pipe_name="clamp_red",
+                      options=list(opts))
+    prm = {'R': 30, 'C': 45}
+    inputs = {'img': np.random.default_rng(7).random((30, 45)).astype(
+        np.float32)}
+    got = emulate.run(p, prm, inputs, tmp_path)["g"]
+    ref = Evaluator(prm, inputs).array(g)
+    # float32 sums of at most 240 values below 1
+    assert np.abs(got - ref).max() <= 240 * 240 * 2.0 ** -24
