@@ -3652,10 +3652,10 @@ class StencilGen(object):
         for d in range(nd):
             w("const int q%d = r_%s_lo%d + j%d;" % (d, nm, d, d))
         w("if (%s) continue;" % " || ".join(
-            "q%d > r_%s_hi%d || q%d < d_%s_lo%d || q%d > d_%s_hi%d" % (
-                d, nm, d, d, fnm, d, d, fnm, d) for d in range(nd)) +
-          "".join(" || q%d > %s" % (d, e)
-                  for d, e in enumerate(self.needed(n)) if e is not None))
+            ["q%d > r_%s_hi%d || q%d < d_%s_lo%d || q%d > d_%s_hi%d" % (
+                d, nm, d, d, fnm, d, d, fnm, d) for d in range(nd)] +
+            ["q%d > %s" % (d, e)
+             for d, e in enumerate(self.needed(n)) if e is not None]))
         self.gen_point(f, n)
         w.close()
 
