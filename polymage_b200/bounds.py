@@ -446,11 +446,19 @@ def excess(a, b, least):
     """The least constant that provably bounds ``a - b`` from above for all
     parameter values (see least_params), or None when the two do not
     compare."""
+    def forms(e):
+        """Enclosures of ``e``, one division deeper each."""
+        out = []
+        for i in range(MAX_QUOTIENTS + 1):
+            q = _enclose(e, i, least)
+            if out and q == out[-1]:
+                break
+            out.append(q)
+        return out
     best = None
-    for i in range(MAX_QUOTIENTS + 1):
-        p = _enclose(a, i, least)
-        for j in range(MAX_QUOTIENTS + 1):
-            q = _enclose(b, j, least)
+    fb = forms(b)
+    for p in forms(a):
+        for q in fb:
             if p[0] == q[0] and (best is None or p[2] - q[1] < best):
                 best = p[2] - q[1]
     return best

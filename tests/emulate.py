@@ -277,7 +277,7 @@ def _device_source(source):
 
 
 def run(pipeline, params, inputs, workdir, shift=0, tma=True, order=0,
-        fill=77, opt="-O1"):
+        fill=77, opt="-O0"):
     """Outputs {name: array} of one device call.  ``shift``: bytes from a
     256-byte boundary to the inputs' bases; ``fill``: the value outputs
     hold before the call; ``order``: 1 runs the threads of a CTA backwards
