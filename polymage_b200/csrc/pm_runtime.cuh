@@ -90,15 +90,19 @@ __device__ __forceinline__ void pm_mbar_inval(uint64_t* bar) {
                : "memory");
 }
 
-// Global loads of a group's kernel body.  A standalone launch reads through
-// the read-only (non-coherent) path: nothing it reads is written while it
-// runs.  A body inside a chain kernel (several groups, one launch, grid
-// barriers between dependent groups) reads data that other CTAs of the same
-// launch wrote before the last barrier, so it bypasses L1 (ld.global.cg).
+// Global loads of a group's kernel body.  A standalone launch may start
+// while the previous kernel of its stream still writes what this one will
+// read (programmatic dependent launch), so it loads by plain ld.global,
+// which stays behind pm_grid_dep_wait: the read-only path (__ldg) asks that
+// the data be constant for the whole run of the kernel, and the compiler may
+// move such loads across the wait.  A body inside a chain kernel (several
+// groups, one launch, grid barriers between dependent groups) reads data
+// that other CTAs of the same launch wrote before the last barrier, so it
+// bypasses L1 (ld.global.cg).
 template <bool CH, typename T>
 __device__ __forceinline__ T pm_ld(const T* p) {
   if constexpr (CH) return __ldcg(p);
-  else return __ldg(p);
+  else return *p;
 }
 
 // Copy of one 4- or 8-byte element to shared memory, zero when `ok` is
