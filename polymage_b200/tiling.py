@@ -1368,6 +1368,15 @@ def _gather_map(pipeline, f, rvars):
 
 
 MAX_CELL_BINS = 64
+# A thread's own bins take shared memory, and with it the threads that hide
+# the sums' latency: the grid-cell form is taken while at least this many
+# stay on an SM.  B200, sums of 2048x2048 values in 8x8 cells, us a call
+# with bins at random / alike in neighbouring rows, against the atomic form:
+# 64 float bins in 256 threads (768 resident) 35 / 35, 27 / 61; 48 double
+# bins in 256 (512 resident) 57 / 56, 42 / 71; 64 double bins in 128 (384)
+# 79 / 74, 70 / 93; in 256 (256 resident) 110 / 104, 44 / 74.
+MIN_CELL_THREADS = 384
+SM_BYTES = 227 * 1024
 
 
 def _cell_map(pipeline, f, fns_all, threads, env):
@@ -1467,10 +1476,14 @@ def plan_reduction(pipeline, comps):
     plan.cells = _cell_map(pipeline, f, fns_all, plan.threads, env)
     if plan.cells is not None:
         (k0, _), _, bins = plan.cells
-        plan.tile = [max(1, plan.tile[0] // k0) * k0, plan.threads]
-        plan.smem_bytes = f.typ.size() * plan.threads * int(
+        nbytes = f.typ.size() * plan.threads * int(
             np.prod(list(bins.values()) or [1]))
-        return plan
+        if nbytes <= int(_option(pipeline, 'smem_budget', SMEM_BUDGET)) and \
+                SM_BYTES // nbytes * plan.threads >= MIN_CELL_THREADS:
+            plan.tile = [max(1, plan.tile[0] // k0) * k0, plan.threads]
+            plan.smem_bytes = nbytes
+            return plan
+        plan.cells = None
     # privatized footprint of one tile, by simulation over a period
     divs = []
     for fns in fns_all:

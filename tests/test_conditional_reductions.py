@@ -6,9 +6,9 @@ import numpy as np
 import pytest
 
 from polymage_b200.compiler import buildPipeline
-from polymage_b200.constructs import (Case, Cast, Condition, Float, Function,
-                                      Image, Int, Interval, Max, Min, Op,
-                                      Parameter, Reduce, Reduction,
+from polymage_b200.constructs import (Case, Cast, Condition, Double, Float,
+                                      Function, Image, Int, Interval, Max,
+                                      Min, Op, Parameter, Reduce, Reduction,
                                       Variable)
 from tests import emulate
 from tests.dsl_eval import Evaluator
@@ -87,3 +87,25 @@ def test_clamped_targets(target, opts, tmp_path):
     ref = Evaluator(prm, inputs).array(g)
     # float32 sums of at most 240 values below 1
     assert np.abs(got - ref).max() <= 240 * 240 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("typ,bins,threads,taken", [
+    (Float, 60, 1024, False), (Double, 64, 512, False),
+    (Double, 64, 256, False), (Double, 64, 128, True),
+    (Float, 64, 256, True), (Float, 28, 1024, True)])
+def test_cells_fit_an_sm(typ, bins, threads, taken):
+    """Per-thread bins that an SM cannot hold, or only for few threads,
+    leave the sum to the atomic form."""
+    img, idx = Image(typ, "img", [R, C]), Image(Int, "idx", [R, C])
+    h = Reduction(([i, j, b], [Interval(Int, 0, R / 8), Interval(
+        Int, 0, C / 8), Interval(Int, 0, bins - 1)]), ([x, y], [
+            Interval(Int, 0, R - 1), Interval(Int, 0, C - 1)]), typ, "h")
+    h.defn = [Case(Condition(b, ">=", 0), Reduce(
+        h(x / 8, y / 8, Cast(Int, idx(x, y))), img(x, y), Op.Sum))]
+    h.default = 0
+    p = buildPipeline([h], param_estimates=[(R, 500), (C, 500)],
+                      tile_sizes=[16, 256], pipe_name="cell_fit",
+                      options=['threads=%d' % threads])
+    plan = p.groups[0].plan
+    assert (plan.cells is not None) == taken
+    assert plan.smem_bytes <= 227 * 1024 and plan.smem_bytes > 0
