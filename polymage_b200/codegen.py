@@ -5149,11 +5149,12 @@ def _chain_limit(pipeline):
 
 
 def _launch_param_bytes(sg):
-    """Upper estimate of sizeof(<k>_launch): tensor maps, parameters,
-    buffer pointers, tile grid, launch fields."""
+    """Upper estimate of sizeof(<k>_launch): tensor maps, precomputed
+    quotients, parameters, buffer pointers, tile grid, launch fields."""
     pg = sg.pg
     na = sg.plan.anchor.ndims
-    desc = 128 * len(sg.stage_nodes) + 8 * (len(pg.params) + len(sg.bufs)) \
+    desc = 128 * len(sg.stage_nodes) + 8 * (
+        len(sg.hoisted) + len(pg.params) + len(sg.bufs)) \
         + 12 * na + 8 + 4 * len(sg.stage_nodes)
     desc = (desc + 63) // 64 * 64
     return desc + 64
@@ -5351,7 +5352,7 @@ def plan_merges(pg, pipeline):
             sg.launch_bounds == pg.stencil_of[i].launch_bounds and
             not (pg.launch_rw[i][1] & rj or pg.launch_rw[i][0] & wj or
                  pg.launch_rw[i][1] & wj) for i in cur) and \
-            sum(_launch_param_bytes(pg.stencil_of[i])
+            sum(_launch_param_bytes(pg.stencil_of[i]) + 4   # and its n[]
                 for i in cur + [j]) <= CHAIN_PARAM_BYTES
         if not fits:
             runs.append(cur)
