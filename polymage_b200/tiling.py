@@ -604,6 +604,18 @@ def plan_stencil(pipeline, comps, tile=None):
                             "anchor %s" % (n.name, anchor.name))
         off = anchor.ndims - n.ndims
         n.owned_map = [off + d for d in range(n.ndims)]
+        for d, dom in enumerate(n.func.domain):
+            k = off + d
+            if _fixed_extent(anchor.domain[k], env) is None:
+                continue
+            # tiles cover the anchor's own range along such a dimension
+            a, b = (_domain_vals(q, env)[j] for q, j in (
+                (anchor, k), (n.func, d)))
+            if _fixed_extent(dom, env) is None or b[0] < a[0] or \
+                    b[1] > a[1]:
+                raise PlanError("live-out %s extends past a dimension of "
+                                "the anchor %s of constant extent" % (
+                                    n.name, anchor.name))
     for n in nodes:
         # materialized consumers read only where their Case holds
         n.case_box = case_box(n.func) if n.role in ('out', 'smem') else None

@@ -51,3 +51,30 @@ def test_values_at_their_place(defn, opts, rows, tmp_path):
     ref = Evaluator(prm, {'img': img}).array(g)
     # float32 sums of three values below 2
     assert np.abs(got - ref).max() <= 4 * 8 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("opts", [('fuse_all',), ()])
+def test_live_out_across_a_dimension_of_bins(opts, tmp_path):
+    """A plane and a volume of bins from one stage: the plane's columns lie
+    along the bins of the volume's tiles, which are fewer."""
+    img = Image(Float, "img", [R, C])
+    z = Variable(Int, "z")
+    rows = Interval(Int, 1, R - 2)
+    f = Function(([x, y], [Interval(Int, 0, R - 1), COLS]), Float, "f")
+    f.defn = [img(x, y) + 1]
+    g2 = Function(([x, y], [rows, COLS]), Float, "g2")
+    g2.defn = [f(x - 1, y) + f(x + 1, y)]
+    g3 = Function(([x, y, z], [rows, COLS, Interval(Int, 0, 4)]), Float,
+                  "g3")
+    g3.defn = [f(x - 1, y) * z + f(x + 1, y)]
+    p = buildPipeline([g2, g3], param_estimates=[(R, 500), (C, 500)],
+                      tile_sizes=[2, 8, 32], pipe_name="plane_volume",
+                      options=list(opts) + ['inline_budget=0'])
+    prm = {'R': 13, 'C': 45}
+    inputs = {'img': np.random.default_rng(4).random((13, 45)).astype(
+        np.float32)}
+    got = emulate.run(p, prm, inputs, tmp_path, fill=0)
+    ev = Evaluator(prm, inputs)
+    for g in (g2, g3):
+        # float32 sums of products below 10
+        assert np.abs(got[g.name] - ev.array(g)).max() <= 4 * 16 * 2.0 ** -24
