@@ -55,18 +55,20 @@ def test_values_at_their_place(defn, opts, rows, tmp_path):
 
 @pytest.mark.parametrize("opts", [('fuse_all',), ()])
 def test_live_out_across_a_dimension_of_bins(opts, tmp_path):
-    """A plane and a volume of bins from one stage: the plane's columns lie
-    along the bins of the volume's tiles, which are fewer."""
+    """A plane and a volume of bins: the plane's columns lie along the bins
+    of the volume's tiles, which are fewer."""
     img = Image(Float, "img", [R, C])
     z = Variable(Int, "z")
     rows = Interval(Int, 1, R - 2)
     f = Function(([x, y], [Interval(Int, 0, R - 1), COLS]), Float, "f")
     f.defn = [img(x, y) + 1]
-    g2 = Function(([x, y], [rows, COLS]), Float, "g2")
-    g2.defn = [f(x - 1, y) + f(x + 1, y)]
+    f2 = Function(([x, y], [rows, COLS]), Float, "f2")
+    f2.defn = [f(x - 1, y) + f(x + 1, y)]
+    g2 = Function(([x, y], [rows, Interval(Int, 1, C - 2)]), Float, "g2")
+    g2.defn = [f2(x, y - 1) + f2(x, y + 1)]
     g3 = Function(([x, y, z], [rows, COLS, Interval(Int, 0, 4)]), Float,
                   "g3")
-    g3.defn = [f(x - 1, y) * z + f(x + 1, y)]
+    g3.defn = [img(x - 1, y) * z + img(x + 1, y)]
     p = buildPipeline([g2, g3], param_estimates=[(R, 500), (C, 500)],
                       tile_sizes=[2, 8, 32], pipe_name="plane_volume",
                       options=list(opts) + ['inline_budget=0'])
