@@ -2143,11 +2143,12 @@ class StencilGen(object):
               "counter.")
             w.open("for (int tile = L.first + pm_bid; tile < L.total; )")
             self.gen_tile_setup("tile")
+            self.gen_smem(None)
             if pdl:
                 # ahead of the restrict-qualified pointers: until here the
                 # previous kernel may write what they point to
                 w("if (!PM_CH) pm_grid_dep_wait();")
-            self.gen_buffers(None)
+            self.gen_buffers()
             if self.stage_nodes:
                 self.gen_issue("pm_bar")
                 self.gen_coop_loads()
@@ -2203,7 +2204,8 @@ class StencilGen(object):
         w.close()
         w.open("")
         self.gen_tile_setup("tile")
-        self.gen_buffers("pm_buf")
+        self.gen_smem("pm_buf")
+        self.gen_buffers()
         self.gen_coop_loads()
         self.gen_wait("pm_bar + pm_buf", "pm_buf", "pm_bar + (pm_buf ^ 1)")
         for f in plan.steps:
@@ -2296,15 +2298,18 @@ class StencilGen(object):
             w("const %s %s = %s%s[%d];" % (
                 typ, nm, "(bool)" if typ == "bool" else "", arr, i))
 
-    def gen_buffers(self, buf):
-        """HBM buffer pointers and shared-memory buffers of the current
-        tile; ``buf``: the copy of the staged inputs (prefetch) or None."""
+    def gen_buffers(self):
+        """HBM buffer pointers of the current tile."""
         pg = self.pg
-        w = pg.w
         for f in self.bufs:
-            w("%s%s* __restrict__ b_%s = D.b_%s;" % (
+            pg.w("%s%s* __restrict__ b_%s = D.b_%s;" % (
                 "" if any(f is n.func for n in self.outs) else "const ",
                 ctype(f.typ), pg.fn(f), pg.fn(f)))
+
+    def gen_smem(self, buf):
+        """Shared-memory buffers of the current tile and their origins;
+        ``buf``: the copy of the staged inputs (prefetch) or None."""
+        w = self.pg.w
         for n in self.plan.nodes:
             if n.in_smem:
                 if n.role == 'stage' and buf is not None:
@@ -3998,9 +4003,9 @@ class StencilGen(object):
         # behind a store that might write what they read, one point's
         # latency after another's.  B200, us a call with stores in place
         # -> here, and what the read-only path took: 8-level pyramid 2048^2
-        # 219 -> 195 (200), camera pipe 1968x2592 34.3 -> 31.1 (33.4).
-        # Points that read shared memory only lose by the longer lives of
-        # their values (unsharp 3x4096x4096 72.5 -> 74.1).
+        # 219 -> 201 (202), camera pipe 1968x2592 34.3 -> 31.9 (33.2).
+        # Points that read shared memory only can lose by the longer lives
+        # of their values (unsharp 3x4096x4096 72.5 -> 74.1).
         late = w
         if any(n2.role == 'global' for n2, _ in self.inline_uses(n)):
             late = W()
