@@ -2647,7 +2647,24 @@ class StencilGen(object):
         memo = self.pg.__dict__.setdefault('_main_parts', {})
         if id(f) not in memo:
             memo[id(f)] = self._main_part(f)
-        return memo[id(f)]
+        return None if self.data_cases(f) else memo[id(f)]
+
+    def data_cases(self, f):
+        """Whether a stage evaluated in registers is read at a
+        data-dependent index along a dimension that its Cases narrow: then
+        they hold at some of its points only, on every tile."""
+        n = self.plan.node_of.get(f)
+        if n is None or n.role != 'inline':
+            return False
+        memo = self.__dict__.setdefault('_data_cases', {})
+        if f not in memo:
+            full = [v for v, k in zip(f.variables, range(n.ndims)) if any(
+                fns[k].kind == 'full' for _, fns in n.uses)]
+            memo[f] = any(
+                any(q is v for q in cond.collect(C.Variable))
+                for cond, _, _ in body_parts(f) if cond is not None
+                for v in full)
+        return memo[f]
 
     def _main_part(self, f):
         parts = body_parts(f)
@@ -2680,18 +2697,6 @@ class StencilGen(object):
                 return b, expr
         return None
 
-    def cases_ok(self, f):
-        """Whether ``f`` can be evaluated without conditions where its main
-        part holds, or by a branch chain over exact boxes."""
-        parts = body_parts(f)
-        if len(parts) == 1 and parts[0][0] is None:
-            return True
-        if self.main_part(f) is not None:
-            return True
-        boxes = part_boxes(f)
-        return len(parts) > 1 and len(boxes) == len(parts) and \
-            all(b[0].exact for b in boxes)
-
     def inline_uses(self, n):
         """(node, [IndexFn lists per dimension]) of every producer that
         the points of step node ``n`` read or evaluate."""
@@ -2703,17 +2708,10 @@ class StencilGen(object):
         return out
 
     def fastable(self, f):
-        """Whether step ``f`` has an unconditional form (see cases_ok):
-        its own Cases and those of every stage it evaluates in
-        registers."""
-        memo = self.__dict__.setdefault('_fastable', {})
-        if f not in memo:
-            n = self.plan.node_of[f]
-            memo[f] = 'guarded' not in self.pg.p.options and \
-                self.cases_ok(f) and all(
-                    n2.role != 'inline' or self.cases_ok(n2.func)
-                    for n2, _ in self.inline_uses(n))
-        return memo[f]
+        """Whether step ``f`` runs its unconditional form where that
+        holds: without conditions on its main part, else with its Cases
+        evaluated but its reads unguarded."""
+        return 'guarded' not in self.pg.p.options
 
     def cover(self, n):
         """{dimension: (offset, count)}: the points of a shared-memory
@@ -3136,6 +3134,20 @@ class StencilGen(object):
         bind = dict(zip(f.variables, args))
         self.emit_cases(f, bind, t, None)
 
+    def selects(self, f):
+        """Whether the unconditional form evaluates all of ``f``'s parts and
+        selects: conditions on data, remainders or several variables, which
+        neighbouring points answer differently (reads are in bounds at
+        every point of that form).  B200, 6000x6000 floats between two 3x3
+        filters, us a call, against a branch for each part and point by
+        point: a 3x3 filter where a value exceeds 0.5 132, 161, 191; rows
+        and columns by parity 124, 127, 205; x >= 10 or y >= 10 129, 220,
+        193; x >= y 131, 166, 166.  Box-shaped Cases are decided alike for
+        whole rows and keep the branches."""
+        boxes = part_boxes(f)
+        return len(boxes) != len(body_parts(f)) or \
+            not all(b[0].exact for b in boxes)
+
     def emit_cases(self, f, bind, target, written_flag):
         """Evaluate ``f``'s definition at the bound point into ``target``
         (already 0); later cases take precedence, as in the reference
@@ -3158,6 +3170,18 @@ class StencilGen(object):
                 if written_flag:
                     w("%s = true;" % written_flag)
                 return
+        if self.inside and self.selects(f):
+            # every part evaluated, the last one that holds taken
+            val = "(%s)0" % ctype(f.typ)
+            held = []
+            for cond, expr, red in parts:
+                held.append("true" if cond is None else ctx.cond(cond, bind))
+                val = "(%s ? (%s)(%s) : %s)" % (
+                    held[-1], ctype(f.typ), ctx.expr(expr, bind), val)
+            w("%s = %s;" % (target, val))
+            if written_flag:
+                w("%s = %s;" % (written_flag, " || ".join(held)))
+            return
         # conditions that read producers are evaluated before the branch
         # chain (their reads are statements)
         texts = {}
@@ -3644,7 +3668,7 @@ class StencilGen(object):
 
     def gen_guarded_loop(self, f, n, ext):
         """One point per iteration over the static box, guarded by the
-        region and the domain: steps without an unconditional form."""
+        region and the domain (options 'guarded', 'no_inside')."""
         pg = self.pg
         w = pg.w
         nm = self.node_name(n)
