@@ -5397,7 +5397,7 @@ def gen_merges(pg, pipeline):
     (``pm_<name>_merge<m>``): its CTAs are the members' tiles one member
     after another.  The 8-level pyramid decimates two images and a mask
     level by level, three short launches a level on three streams; merged
-    it takes 16 launches on one stream instead of 30, which the host
+    it takes 15 launches on one stream instead of 30, which the host
     issues about 4.4 us apart (B200, us a call, 256^2 119 -> 85, 1001x1403
     135 -> 131, 2048^2 207 -> 201)."""
     runs = plan_merges(pg, pipeline)
