@@ -3418,7 +3418,8 @@ class StencilGen(object):
         # far tiles, 8 consecutive along every parametric anchor dim (a
         # full period of any residue mod 8 of a region origin whose scale
         # factors divide the tile sizes; others show up as several values)
-        # and the actual ones along dims of constant extent
+        # and the actual ones along dims between constant bounds; where the
+        # grid starts at a parameter, origins of every residue
         axes = []
         for k, t in enumerate(plan.tile):
             dom = plan.anchor.domain[k]
@@ -3426,13 +3427,22 @@ class StencilGen(object):
                 axes.append(np.arange(eval_int(dom.lowerBound, env),
                                       eval_int(dom.upperBound, env) + 1, t,
                                       dtype=np.int64))
+            elif glo[k] is not None:
+                axes.append(glo[k] + (big + np.arange(8, dtype=np.int64)) * t)
             else:
-                axes.append((glo[k] if glo[k] is not None else 0) +
-                            (big + np.arange(8, dtype=np.int64)) * t)
-        grids = np.meshgrid(*axes, indexing='ij')
+                axes.append(big * t + np.arange(8, dtype=np.int64))
+        # and a row of tiles through a whole period of the divisors met,
+        # along all dims at once
+        count = min(8 * max(plan.period, 1), 4096)
+        far = [a[0] + np.arange(count, dtype=np.int64) * (
+            1 if glo[k] is None else plan.tile[k])
+            if not self.const_dim(plan.anchor, k) else
+            a[np.arange(count) % len(a)] for k, a in enumerate(axes)]
+        grids = [np.concatenate([g.ravel(), f]) for g, f in zip(
+            np.meshgrid(*axes, indexing='ij'), far)]
         box = []
         for k, t in enumerate(plan.tile):
-            lo = grids[k].ravel()
+            lo = grids[k]
             hi = lo + t - 1
             if self.const_dim(plan.anchor, k):
                 hi = np.minimum(hi, axes[k][0] + eval_int(

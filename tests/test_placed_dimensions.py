@@ -80,3 +80,28 @@ def test_live_out_across_a_dimension_of_bins(opts, tmp_path):
     for g in (g2, g3):
         # float32 sums of products below 10
         assert np.abs(got[g.name] - ev.array(g)).max() <= 4 * 16 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("rows", [9, 40, 43])
+@pytest.mark.parametrize("rblock", [2, 4])
+def test_rows_that_start_at_a_parameter(rows, rblock, tmp_path):
+    """Tiles start at R / 4 + 5: the row that a block starts at has no
+    known remainder, so the halves of its index do not fold."""
+    img = Image(Float, "img", [R + 8, C + 8])
+    cols = Interval(Int, 4, 2 * C - 4)
+    f = Function(([x, y], [Interval(Int, 2, 2 * R), cols]), Float, "f")
+    f.defn = [img(x / 2 - 1, y / 2) + img(x / 2, y / 2)]
+    g = Function(([x, y], [Interval(Int, R / 4 + 5, 3 * R),
+                           Interval(Int, 8, 3 * C)]), Float, "g")
+    g.defn = [f(x / 2, y / 2) + f(x / 2 + 1, y / 2 + 1) +
+              f(x / 2, y / 2 + 1)]
+    p = buildPipeline([g], param_estimates=[(R, 500), (C, 500)],
+                      tile_sizes=[16, 32], pipe_name="start_rows",
+                      options=['inline_budget=0', 'rblock=%d' % rblock])
+    prm = {'R': rows, 'C': 25}
+    inputs = {'img': np.random.default_rng(rows).random(
+        (rows + 8, 33)).astype(np.float32)}
+    got = emulate.run(p, prm, inputs, tmp_path)["g"]
+    # float32 sums of six values below 1
+    assert np.abs(got - Evaluator(prm, inputs).array(g)).max() <= \
+        8 * 8 * 2.0 ** -24
