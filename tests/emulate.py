@@ -165,7 +165,8 @@ static void pm_cp_async_wait() {}
 // a chain kernel runs as one CTA here, so its own barriers order its phases
 static bool pm_grid_sync(unsigned*, unsigned, unsigned*) { __syncthreads(); return true; }
 static void pm_mbar_arrive_expect_tx(uint64_t*, uint32_t b) { emu_expect += b; }
-static bool pm_mbar_wait(uint64_t*, uint32_t, unsigned*) { return true; }
+// (copies are done when they are issued; the bytes announced have to match)
+static bool pm_mbar_wait(uint64_t*, uint32_t, unsigned*) { assert(emu_expect == emu_got); return true; }
 template <bool CH, typename T> static void pm_copy(T* dst, const T* src, bool ok) { *dst = ok ? *src : (T)0; }
 static void emu_tma(void* dst, const CUtensorMap* m, const int* c) {
   emu_map e;
